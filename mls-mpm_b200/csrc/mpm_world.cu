@@ -153,8 +153,8 @@ __device__ __forceinline__ void bin_cell(const SceneDesc& sd, float px, float py
 // Appends a scene's particles at positions [pos0, pos0 + n) with their keys.
 __global__ void k_import(WorldView v, uint32_t scene, uint32_t pos0, const float4* __restrict__ pos,
                          const float4* __restrict__ vel, const float* __restrict__ aff,
-                         const float* __restrict__ mass, float4* __restrict__ posm, float4* __restrict__ velid,
-                         float* __restrict__ aff_out, uint32_t n) {
+                         const float* __restrict__ mass, float4* __restrict__ posm, float4* __restrict__ rows,
+                         uint32_t* __restrict__ ids, uint32_t n) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const SceneDesc& sd = v.scenes[scene];
@@ -163,9 +163,13 @@ __global__ void k_import(WorldView v, uint32_t scene, uint32_t pos0, const float
     const float4 q = pos[i];
     const float4 vv = vel ? vel[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     posm[p] = make_float4(q.x, q.y, q.z, mass[i]);
-    velid[p] = make_float4(vv.x, vv.y, vv.z, __uint_as_float(sd.id_base + i));
+    ids[p] = sd.id_base + i;
+    const float v3[3] = {vv.x, vv.y, vv.z};
 #pragma unroll
-    for (int e = 0; e < 9; ++e) aff_out[e * plane + p] = aff ? aff[9ull * i + e] : 0.0f;
+    for (int c = 0; c < 3; ++c) {
+        const float* a = aff + 9ull * i + 3 * c;
+        rows[c * plane + p] = aff ? make_float4(a[0], a[1], a[2], v3[c]) : make_float4(0.0f, 0.0f, 0.0f, v3[c]);
+    }
     int32_t cx, cy, cz;
     bin_cell(sd, q.x, q.y, q.z, cx, cy, cz);
     v.key[p] = sd.cell_base + local_cell(sd, cx, cy, cz);
@@ -173,12 +177,11 @@ __global__ void k_import(WorldView v, uint32_t scene, uint32_t pos0, const float
 }
 
 // Drops a scene's particles: their positions become holes.
-__global__ void k_remove(WorldView v, const float4* __restrict__ velid, uint32_t id0, uint32_t n) {
+__global__ void k_remove(WorldView v, const uint32_t* __restrict__ ids, uint32_t id0, uint32_t n) {
     const uint32_t total = min(v.ctrl->total_pos, v.npos);
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < total; p += gridDim.x * blockDim.x) {
         if (v.key[p] == kHole) continue;
-        const uint32_t id = __float_as_uint(velid[p].w);
-        if (id - id0 < n) v.key[p] = kHole;
+        if (ids[p] - id0 < n) v.key[p] = kHole;
     }
 }
 
@@ -191,24 +194,24 @@ __global__ void k_extend(WorldView v, uint32_t end) {
 }
 
 // Writes a scene's particles to reference-layout buffers by local id.
-__global__ void k_export(WorldView v, const float4* __restrict__ posm, const float4* __restrict__ velid,
-                         const float* __restrict__ aff, const float* __restrict__ dens, uint32_t id0, uint32_t n,
+__global__ void k_export(WorldView v, const float4* __restrict__ posm, const float4* __restrict__ rows,
+                         const uint32_t* __restrict__ ids, const float* __restrict__ dens, uint32_t id0, uint32_t n,
                          float4* __restrict__ pos, float4* __restrict__ vel, float* __restrict__ aff_out,
                          float* __restrict__ mass, float* __restrict__ dens_out) {
     const uint32_t total = min(v.ctrl->total_pos, v.npos);
     const size_t plane = v.npos;
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < total; j += gridDim.x * blockDim.x) {
         if (v.key[j] == kHole) continue;
-        const float4 vv = velid[j];
-        const uint32_t id = __float_as_uint(vv.w) - id0;
+        const uint32_t id = ids[j] - id0;
         if (id >= n) continue;
-        const float4 p = posm[j];
+        const float4 p = posm[j], r0 = rows[j], r1 = rows[plane + j], r2 = rows[2 * plane + j];
         pos[id] = make_float4(p.x, p.y, p.z, 0.0f);
-        vel[id] = make_float4(vv.x, vv.y, vv.z, 0.0f);
+        vel[id] = make_float4(r0.w, r1.w, r2.w, 0.0f);
         mass[id] = p.w;
         if (dens_out) dens_out[id] = dens[j];
+        const float a[9] = {r0.x, r0.y, r0.z, r1.x, r1.y, r1.z, r2.x, r2.y, r2.z};
 #pragma unroll
-        for (int e = 0; e < 9; ++e) aff_out[9ull * id + e] = aff[e * plane + j];
+        for (int e = 0; e < 9; ++e) aff_out[9ull * id + e] = a[e];
     }
 }
 
@@ -713,10 +716,13 @@ __device__ __forceinline__ void copy_scene_async_one(const WorldView& v, uint32_
 // True when the particle's 3x3x3 stencil lies in the chunk's halo box and in
 // the grid (then shared-memory accumulation / gathering is exact); otherwise
 // the particle takes the direct path with the reference's indexing.
+__device__ __forceinline__ bool in_halo(int32_t cx, int32_t cy, int32_t cz, const ChunkHdr& h, const SceneDesc& sd) {
+    return cx - 1 >= h.ox && cy - 1 >= h.oy && cz - 1 >= h.oz && cx + 1 < h.ox + h.hx && cy + 1 < h.oy + h.hy &&
+           cz + 1 < h.oz + h.hz && cx >= 1 && cy >= 1 && cz >= 1 && cx + 1 < (int32_t)sd.X &&
+           cy + 1 < (int32_t)sd.Y && cz + 1 < (int32_t)sd.Z;
+}
 __device__ __forceinline__ bool in_halo(const PW& w, const ChunkHdr& h, const SceneDesc& sd) {
-    return w.cx - 1 >= h.ox && w.cy - 1 >= h.oy && w.cz - 1 >= h.oz && w.cx + 1 < h.ox + h.hx &&
-           w.cy + 1 < h.oy + h.hy && w.cz + 1 < h.oz + h.hz && w.cx >= 1 && w.cy >= 1 && w.cz >= 1 &&
-           w.cx + 1 < (int32_t)sd.X && w.cy + 1 < (int32_t)sd.Y && w.cz + 1 < (int32_t)sd.Z;
+    return in_halo(w.cx, w.cy, w.cz, h, sd);
 }
 
 // Shared halo arrays use the strides of the largest box (a tile plus its
@@ -730,19 +736,28 @@ __device__ __forceinline__ int halo_base(const ChunkHdr& h, int32_t cx, int32_t 
     return (cz - 1 - h.oz) * kHXY + (cy - 1 - h.oy) * kHX + (cx - 1 - h.ox);
 }
 
-// Slots of the halo arrays that the chunk's box spans: [0, halo_span(h)).
-// Loops over them divide by compile-time strides only.
-__device__ __forceinline__ int halo_span(const ChunkHdr& h) { return h.hz * kHXY; }
+// What the halo loops need of a scene.
+struct GridDims {
+    uint32_t X, Y, Z, cell_base;
+};
+__device__ __forceinline__ GridDims grid_dims(const SceneDesc& sd) { return GridDims{sd.X, sd.Y, sd.Z, sd.cell_base}; }
 
-// Slot s as a cell of the chunk's box inside the grid: its scene-local cell,
-// or false for a slot outside the box or a box cell outside the grid.
-__device__ __forceinline__ bool halo_cell(const ChunkHdr& h, const SceneDesc& sd, int s, uint32_t& cell) {
-    const int dz = s / kHXY, r = s - dz * kHXY, dy = r / kHX, dx = r - dy * kHX;
-    if (dx >= h.hx || dy >= h.hy) return false;
-    const int32_t x = h.ox + dx, y = h.oy + dy, z = h.oz + dz;
-    if (x < 0 || y < 0 || z < 0 || x >= (int32_t)sd.X || y >= (int32_t)sd.Y || z >= (int32_t)sd.Z) return false;
-    cell = local_cell(sd, x, y, z);
-    return true;
+// Calls f(halo slot, scene-local cell) for every cell of the chunk's box that
+// lies in the grid (a particle that uses the halo has its stencil there), one
+// thread per (x, y) column of the largest box: the coordinates and the cell
+// are worked out once for the column instead of once for each slot.
+template <uint32_t kT, class F>
+__device__ __forceinline__ void halo_columns(const ChunkHdr& h, const GridDims& sd, F&& f) {
+    for (uint32_t col = threadIdx.x; col < (uint32_t)kHXY; col += kT) {
+        const int dy = (int)(col / (uint32_t)kHX), dx = (int)col - dy * kHX;
+        const int32_t x = h.ox + dx, y = h.oy + dy;
+        if (dx >= h.hx || dy >= h.hy || (uint32_t)x >= sd.X || (uint32_t)y >= sd.Y) continue;
+        const int z0 = max(0, -h.oz), z1 = min(h.hz, (int)sd.Z - h.oz);
+        const uint32_t slab = sd.X * sd.Y;
+        uint32_t cell = ((uint32_t)(h.oz + z0) * sd.Y + (uint32_t)y) * sd.X + (uint32_t)x;
+        int s = z0 * kHXY + (int)col;
+        for (int dz = z0; dz < z1; ++dz, cell += slab, s += kHXY) f(s, cell);
+    }
 }
 
 // The 27 P2G_MASS contributions of one particle into the shared halo at base
@@ -817,7 +832,6 @@ __global__ void __launch_bounds__(kChunkThreads) k_p2g_mass_chunks(WorldView v, 
             const uint32_t p = h.first + chunk_slot<kC>(r);
             q[r] = p < h.end ? posm[v.perm[p]] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
-        const int hn = halo_span(h);
         const SceneDesc& sd = ssd[sb];
 #pragma unroll
         for (int r = 0; r < kPer; ++r) {
@@ -864,13 +878,12 @@ __global__ void __launch_bounds__(kChunkThreads) k_p2g_mass_chunks(WorldView v, 
             }
         }
         int32_t* scm = cm + sd.cell_base;
-        for (int i = threadIdx.x; i < hn; i += blockDim.x) {
+        halo_columns<kChunkThreads>(h, grid_dims(sd), [&](int i, uint32_t cell) {
             const int32_t a = acc[i];
-            if (a == 0) continue;
+            if (a == 0) return;
             acc[i] = 0;
-            uint32_t cell;
-            if (halo_cell(h, sd, i, cell)) atomicAdd(&scm[cell], a);
-        }
+            atomicAdd(&scm[cell], a);
+        });
         if (threadIdx.x == 0) {
             cp_async_wait();
             ss_nxt = h.scene;   // after the swap ssd[sb ^ 1] holds this chunk's scene
@@ -1262,10 +1275,10 @@ __device__ __forceinline__ float density_shared(const PW& w, const float* m) {
 
 // P2G_MOM for one particle whose inputs are loaded.
 __device__ __forceinline__ void mom_particle(const WorldView& v, const ChunkHdr& h, const SceneDesc& sd, bool valid,
-                                             uint32_t p, const float4 pm, const float4 vi, const float* a,
+                                             const float4 pm, const float4 r0, const float4 r1, const float4 r2,
                                              const float* mh, int32_t (*acc)[kHaloCells],
                                              const float* __restrict__ scmf, int32_t* __restrict__ smv,
-                                             float* __restrict__ dens, uint32_t* __restrict__ health) {
+                                             float* dens, uint32_t* __restrict__ health) {
     const uint32_t X = sd.X, SLICE = sd.X * sd.Y, G = sd.G;
     const PW w = particle_weights(pm.x, pm.y, pm.z);
     const bool fast = valid && in_halo(w, h, sd);
@@ -1284,11 +1297,11 @@ __device__ __forceinline__ void mom_particle(const WorldView& v, const ChunkHdr&
                     density += w.wx[i] * w.wy[jj] * w.wz[k] * cmass;
                 }
     }
-    if (valid) dens[p] = density;
+    if (valid) *dens = density;
     const bool live = valid && density > 1e-8f;   // shaders.js:315
     // stress (shaders.js:325-338)
     const float rest = sd.P.rest_density;
-    const MomIn in{vi.x, vi.y, vi.z, pm.w, a[0], a[1], a[2], a[3], a[4], a[5], a[6], a[7], a[8]};
+    const MomIn in{r0.w, r1.w, r2.w, pm.w, r0.x, r0.y, r0.z, r1.x, r1.y, r1.z, r2.x, r2.y, r2.z};
     const float vol = __fdiv_rn(in.m, fmaxf(density, rest * 0.15f));
     float pressure = sd.P.stiffness * (eos_pow(__fdiv_rn(density, rest), sd.P.eos_power) - 1.0f);
     const float pFloor = density > rest * kCohesionGate ? kCohesionPressure : 0.0f;
@@ -1349,32 +1362,32 @@ __device__ __forceinline__ void mom_particle(const WorldView& v, const ChunkHdr&
 // accumulators are zeroed by the flush that reads them.
 __device__ __forceinline__ void stage_masses_async(const WorldView& v, const ChunkHdr& hh,
                                                    const float* __restrict__ cmf, float* buf) {
-    const SceneDesc& nsd = v.scenes[hh.scene];
-    const float* src = cmf + nsd.cell_base;
-    const int hn = halo_span(hh);
-    for (int i = threadIdx.x; i < hn; i += blockDim.x) {
-        uint32_t cell;
-        const bool in = halo_cell(hh, nsd, i, cell);
-        cp_async4z(buf + i, in ? (const void*)(src + cell) : (const void*)src, in ? 4u : 0u);
-    }
+    const GridDims g = grid_dims(v.scenes[hh.scene]);
+    const float* src = cmf + g.cell_base;
+    halo_columns<kChunkThreads>(hh, g, [&](int s, uint32_t cell) { cp_async4z(buf + s, src + cell, 4u); });
 }
 
+// One particle's inputs: four 16-byte words.  A warp's lanes spread over the
+// chunk, so each of its loads touches up to 32 lines whatever its width: with
+// the velocity and the affine's nine planes as loads of their own (eleven) the
+// L1 data path was 70% busy and bound the kernel together with its issue slots
+// (1M dam break in motion 96 -> 90 us, 8M 661 -> 615 us with four).
+struct MomLoad {
+    float4 pm, row[3];   // x, y, z, mass; affine row and velocity of each axis
+};
 __device__ __forceinline__ void mom_load(const WorldView& v, uint32_t p, bool valid, const float4* __restrict__ posm,
-                                         const float4* __restrict__ velid, const float* __restrict__ aff,
-                                         size_t plane, float4& pm, float4& vi, float* a) {
-    const uint32_t slot = valid ? v.perm[p] : 0u;
-    if (valid) {
-        pm = posm[slot];
-        vi = velid[slot];
-    }
-#pragma unroll
-    for (int e = 0; e < 9; ++e) a[e] = valid ? aff[e * plane + slot] : 0.0f;
+                                         const float4* __restrict__ rows, size_t plane, MomLoad& in) {
+    if (!valid) return;
+    const uint32_t slot = v.perm[p];
+    in.pm = posm[slot];
+    in.row[0] = rows[slot];
+    in.row[1] = rows[plane + slot];
+    in.row[2] = rows[2 * plane + slot];
 }
 
 template <uint32_t kC>
 __global__ void __launch_bounds__(kChunkThreads, MPM_MOM_MINB) k_p2g_mom_chunks(WorldView v, const float4* __restrict__ posm,
-                                                                   const float4* __restrict__ velid,
-                                                                   const float* __restrict__ aff,
+                                                                   const float4* __restrict__ rows,
                                                                    const float* __restrict__ cmf,
                                                                    int32_t* __restrict__ mv,
                                                                    float* __restrict__ dens) {
@@ -1407,9 +1420,8 @@ __global__ void __launch_bounds__(kChunkThreads, MPM_MOM_MINB) k_p2g_mom_chunks(
     // the first particle's inputs
     uint32_t p = hdr[0].first + chunk_slot<kC>(0);
     bool valid = p < hdr[0].end;
-    float4 pm = make_float4(0.0f, 0.0f, 0.0f, 0.0f), vi = pm;
-    float a[9];
-    mom_load(v, p, valid, posm, velid, aff, plane, pm, vi, a);
+    MomLoad in{};
+    mom_load(v, p, valid, posm, rows, plane, in);
     cp_async_wait();
     __syncthreads();
     int b = 0;
@@ -1447,35 +1459,28 @@ __global__ void __launch_bounds__(kChunkThreads, MPM_MOM_MINB) k_p2g_mom_chunks(
                 pn = next_first + chunk_slot<kC>(0);
                 vn = has_next && pn < next_end;
             }
-            float4 pmn = make_float4(0.0f, 0.0f, 0.0f, 0.0f), vin = pmn;
-            float an[9];
-            mom_load(v, pn, vn, posm, velid, aff, plane, pmn, vin, an);
-            mom_particle(v, h, sd, valid, p, pm, vi, a, mh[b], acc, scmf, smv, dens, v.health + h.scene);
+            MomLoad next{};
+            mom_load(v, pn, vn, posm, rows, plane, next);
+            mom_particle(v, h, sd, valid, in.pm, in.row[0], in.row[1], in.row[2], mh[b], acc, scmf, smv, dens + p,
+                         v.health + h.scene);
             p = pn;
             valid = vn;
-            pm = pmn;
-            vi = vin;
-#pragma unroll
-            for (int e = 0; e < 9; ++e) a[e] = an[e];
+            in = next;
         }
         __syncthreads();
         // hdr[b] is free: the header two chunks ahead goes there
         if (threadIdx.x == 0 && nxt2 < nch) hdr[b] = unpack_header(nh0, nh1);
-        const int hn = halo_span(h);
-        for (int i = threadIdx.x; i < hn; i += blockDim.x) {
-            const int32_t a0 = acc[0][i], a1 = acc[1][i], a2 = acc[2][i];
-            if ((a0 | a1 | a2) == 0) continue;
-            acc[0][i] = 0;
-            acc[1][i] = 0;
-            acc[2][i] = 0;
-            uint32_t cell;
-            if (halo_cell(h, sd, i, cell)) {
-                int32_t* d = smv + 3ull * cell;
-                if (a0) atomicAdd(d + 0, a0);
-                if (a1) atomicAdd(d + 1, a1);
-                if (a2) atomicAdd(d + 2, a2);
-            }
-        }
+        halo_columns<kChunkThreads>(h, grid_dims(sd), [&](int s, uint32_t cell) {
+            const int32_t a0 = acc[0][s], a1 = acc[1][s], a2 = acc[2][s];
+            if ((a0 | a1 | a2) == 0) return;
+            acc[0][s] = 0;
+            acc[1][s] = 0;
+            acc[2][s] = 0;
+            int32_t* d = smv + 3ull * cell;
+            atomicAdd(d + 0, a0);
+            atomicAdd(d + 1, a1);
+            atomicAdd(d + 2, a2);
+        });
         cp_async_wait();
         __syncthreads();
         b ^= 1;
@@ -1680,8 +1685,8 @@ __device__ MPM_G2P_RARE G2PSum g2p_gather_direct(const PW w, const float4 q, con
 // diffuse spawn staging.
 struct G2POut {
     float4* posm;
-    float4* velid;
-    float* aff;
+    float4* rows;
+    uint32_t* ids;
     size_t plane;
     uint32_t* key;
     uint32_t* rank;
@@ -1704,16 +1709,17 @@ struct G2POut {
 // its new binning cell (the caller stores it at rank[p], as late as it can,
 // so the atomic's round trip overlaps later work).
 __device__ __forceinline__ uint32_t g2p_store(const G2POut& o, const SceneDesc& sd, uint32_t p, const float4 q,
-                                              const float4 vi, float density, float gvx, float gvy, float gvz,
+                                              uint32_t gid, float density, float gvx, float gvy, float gvz,
                                               const float* B, const RefOut& ro, bool mirror) {
-#pragma unroll
-    for (int e = 0; e < 9; ++e) o.aff[e * o.plane + p] = B[e] * 4.0f;
     f3 np, nv;
     g2p_finish(q, gvx, gvy, gvz, sd.P, sd.W, np, nv);
     o.posm[p] = make_float4(np.x, np.y, np.z, q.w);
-    o.velid[p] = make_float4(nv.x, nv.y, nv.z, vi.w);
+    o.rows[p] = make_float4(B[0] * 4.0f, B[1] * 4.0f, B[2] * 4.0f, nv.x);
+    o.rows[o.plane + p] = make_float4(B[3] * 4.0f, B[4] * 4.0f, B[5] * 4.0f, nv.y);
+    o.rows[2 * o.plane + p] = make_float4(B[6] * 4.0f, B[7] * 4.0f, B[8] * 4.0f, nv.z);
+    o.ids[p] = gid;
     if (mirror) {   // particle_pos/vel (shaders.js:703-704) and particle_density (shaders.js:314) by id
-        const uint32_t id = __float_as_uint(vi.w) - sd.id_base;
+        const uint32_t id = gid - sd.id_base;
         if (id < sd.n) {
 #if MPM_MIRROR_KEEP
             // the scattered 16- and 4-byte writes by id fill 32-byte sectors
@@ -1756,7 +1762,7 @@ __device__ __forceinline__ uint32_t g2p_store(const G2POut& o, const SceneDesc& 
         if ((threadIdx.x & 31u) == (uint32_t)(__ffs(same) - 1)) atomicOr(&o.tile_flags[t], 1u);
     }
     if (o.gen) {
-        const uint32_t id = __float_as_uint(vi.w) - sd.id_base;
+        const uint32_t id = gid - sd.id_base;
         // spawn_record's first test (shaders.js:806), checked inline
         if (id < sd.n && density > 0.0f && density <= o.bubble_min) {
             const SpawnPre pre = spawn_pre(nv, q.w, density, sd, o.pressure_threshold);
@@ -1770,12 +1776,12 @@ __device__ __forceinline__ uint32_t g2p_store(const G2POut& o, const SceneDesc& 
 // G2P of a particle whose stencil leaves the halo box or the grid (rare): the
 // reference's linear stencil index with a bounds guard, then the epilogue.
 __device__ __noinline__ void g2p_direct_particle(const G2POut o, const SceneDesc* sdp, uint32_t p, const float4 q,
-                                                 const float4 vi, const float4* __restrict__ vel4, const RefOut ro,
+                                                 uint32_t gid, const float4* __restrict__ vel4, const RefOut ro,
                                                  bool mirror) {
     const SceneDesc& sd = *sdp;
     const PW w = particle_weights(q.x, q.y, q.z);
     const G2PSum r = g2p_gather_direct(w, q, vel4, sd.X, sd.Y, sd.G);
-    o.rank[p] = g2p_store(o, sd, p, q, vi, o.dens[p], r.gv[0], r.gv[1], r.gv[2], r.B, ro, mirror);
+    o.rank[p] = g2p_store(o, sd, p, q, gid, o.dens[p], r.gv[0], r.gv[1], r.gv[2], r.B, ro, mirror);
 }
 
 #if MPM_G2P_PACKED
@@ -1822,12 +1828,12 @@ __device__ __forceinline__ void g2p_gather_packed(const PW& w, const float4 q, c
 
 template <uint32_t kC>
 __global__ void __launch_bounds__(kChunkThreads, MPM_G2P_MINB) k_g2p_chunks(WorldView v, const float4* __restrict__ posm,
-                                                              const float4* __restrict__ velid,
+                                                              const uint32_t* __restrict__ ids_in,
                                                               const float4* __restrict__ vel4,
                                                               const float* __restrict__ cmf,
                                                               float4* __restrict__ posm_out,
-                                                              float4* __restrict__ velid_out,
-                                                              float* __restrict__ aff_out, DiffuseView dv,
+                                                              float4* __restrict__ rows_out,
+                                                              uint32_t* __restrict__ ids_out, DiffuseView dv,
                                                               RefOut ro) {
     constexpr int kPer = kC / kChunkThreads;
     __shared__ float4 vh[kHaloCells];   // staged grid velocities (x, y, z, 0)
@@ -1869,27 +1875,23 @@ __global__ void __launch_bounds__(kChunkThreads, MPM_G2P_MINB) k_g2p_chunks(Worl
         const SceneDesc& sd = ssd[sb];
         // this thread's particles, in flight while the halo is staged
         float4 qs[kPer];
-        float ids[kPer], dns[kPer];
+        uint32_t ids[kPer];
+        float dns[kPer];
 #pragma unroll
         for (int r = 0; r < kPer; ++r) {
             const uint32_t p = h.first + r * kChunkThreads + threadIdx.x;
             qs[r] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            ids[r] = 0.0f;
+            ids[r] = 0u;
             dns[r] = 0.0f;
             if (p < h.end) {
                 const uint32_t slot = v.perm[p];
                 qs[r] = posm[slot];
-                ids[r] = velid[slot].w;
+                ids[r] = ids_in[slot];
                 dns[r] = v.dens[p];
             }
         }
-        const int hn = halo_span(h);
         const float4* svel = vel4 + sd.cell_base;
-        for (int i = threadIdx.x; i < hn; i += blockDim.x) {
-            uint32_t cell;
-            const bool in = halo_cell(h, sd, i, cell);
-            cp_async16(&vh[i], in ? (const void*)(svel + cell) : (const void*)svel, in ? 16u : 0u);
-        }
+        halo_columns<kChunkThreads>(h, grid_dims(sd), [&](int i, uint32_t cell) { cp_async16(&vh[i], svel + cell, 16u); });
         cp_async_wait();
         __syncthreads();
         // every thread holds this chunk's header: the next one can replace it
@@ -1903,7 +1905,7 @@ __global__ void __launch_bounds__(kChunkThreads, MPM_G2P_MINB) k_g2p_chunks(Worl
         }
         const bool spawn_scene = dv.enabled && h.scene == dv.scene;
         const bool mirror = ro.enabled && h.scene == ro.scene;
-        const G2POut out{posm_out, velid_out, aff_out, plane, v.key, v.rank, v.cell_count, v.tile_flags, v.dens,
+        const G2POut out{posm_out, rows_out, ids_out, plane, v.key, v.rank, v.cell_count, v.tile_flags, v.dens,
                          cmf + sd.cell_base, spawn_scene ? dv.gen : nullptr, bubble_min, pressure_threshold,
                          ke_threshold, dv.staging, dv.spawn_bits, dv.group_counts};
 #pragma unroll 1
@@ -1911,10 +1913,9 @@ __global__ void __launch_bounds__(kChunkThreads, MPM_G2P_MINB) k_g2p_chunks(Worl
             const uint32_t p = h.first + r * kChunkThreads + threadIdx.x;
             if (p >= h.end) break;
             const float4 q = qs[r];
-            const float4 vi = make_float4(0.0f, 0.0f, 0.0f, ids[r]);
             const PW w = particle_weights(q.x, q.y, q.z);
             if (!in_halo(w, h, sd)) {
-                g2p_direct_particle(out, &sd, p, q, vi, svel, ro, mirror);
+                g2p_direct_particle(out, &sd, p, q, ids[r], svel, ro, mirror);
                 continue;
             }
             float gvx = 0.0f, gvy = 0.0f, gvz = 0.0f;
@@ -1948,7 +1949,7 @@ __global__ void __launch_bounds__(kChunkThreads, MPM_G2P_MINB) k_g2p_chunks(Worl
                 }
             }
 #endif
-            const uint32_t rk = g2p_store(out, sd, p, q, vi, dns[r], gvx, gvy, gvz, B, ro, mirror);
+            const uint32_t rk = g2p_store(out, sd, p, q, ids[r], dns[r], gvx, gvy, gvz, B, ro, mirror);
             // the previous particle's rank: its atomic has long returned
             if (pend_p != kHole) v.rank[pend_p] = pend_rank;
             pend_p = p;
@@ -1992,8 +1993,8 @@ template <class F> static void world_arrays(World& w, F&& f) {
     const size_t NG = (T + 1023) / 1024 + 1;
     for (int b = 0; b < 2; ++b) {
         f(w.posm[b], P * 16);
-        f(w.velid[b], P * 16);
-        f(w.aff[b], P * 36);
+        f(w.rows[b], P * 48);
+        f(w.pid[b], P * 4);
         f(w.grid_i32[b], C * 16);
     }
     f(w.dens, P * 4);
@@ -2276,7 +2277,7 @@ cudaError_t world_add_scene(World& w, uint32_t X, uint32_t Y, uint32_t Z, const 
         const WorldView v = w.view();
         k_extend<<<std::max(1u, std::min<uint32_t>(cdiv(h_total, 256), w.pos_blocks)), 256, 0, w.stream>>>(v, h_total);
         k_import<<<cdiv(n, 256), 256, 0, w.stream>>>(v, (uint32_t)slot, h_total, pos, vel, aff, mass,
-                                                     w.posm[w.cur], w.velid[w.cur], w.aff[w.cur], n);
+                                                     w.posm[w.cur], w.rows[w.cur], w.pid[w.cur], n);
         k_set_total<<<1, 1, 0, w.stream>>>(w.ctrl, h_total + n);
         w.launches += 3;
         w.tbl_outside[w.cur] = true;
@@ -2317,7 +2318,7 @@ cudaError_t world_remove_scene(World& w, int slot) {
     SceneRec& r = w.scenes[slot];
     const WorldView v = w.view();
     if (r.n) {
-        k_remove<<<w.pos_blocks, 256, 0, w.stream>>>(v, w.velid[w.cur], r.id_base, r.n);
+        k_remove<<<w.pos_blocks, 256, 0, w.stream>>>(v, w.pid[w.cur], r.id_base, r.n);
         w.launches++;
         w.tbl_outside[w.cur] = true;
     }
@@ -2359,7 +2360,7 @@ cudaError_t world_export_scene(World& w, int slot, float4* pos, float4* vel, flo
     const SceneRec& r = w.scenes[slot];
     if (!r.live || r.n == 0) return cudaSuccess;
     const WorldView v = w.view();
-    k_export<<<w.pos_blocks, 256, 0, w.stream>>>(v, w.posm[w.cur], w.velid[w.cur], w.aff[w.cur], w.dens,
+    k_export<<<w.pos_blocks, 256, 0, w.stream>>>(v, w.posm[w.cur], w.rows[w.cur], w.pid[w.cur], w.dens,
                                                       r.id_base, r.n, pos, vel, aff, mass,
                                                       w.dens_valid ? dens : nullptr);
     w.launches++;
@@ -2450,11 +2451,11 @@ static cudaError_t enqueue_substep(World& w, Scene* ds, const RefOut& ro, bool t
     {
         Phase ph(prof, MPM_PHASE_P2G_MOM);
         if (w.chunk == kChunkSmall)
-            k_p2g_mom_chunks<kChunkSmall><<<w.item_blocks, kChunkThreads, 0, st>>>(v, w.posm[cur], w.velid[cur],
-                                                                                 w.aff[cur], w.cmf, mv, w.dens);
+            k_p2g_mom_chunks<kChunkSmall><<<w.item_blocks, kChunkThreads, 0, st>>>(v, w.posm[cur], w.rows[cur], w.cmf, mv,
+                                                                                 w.dens);
         else
-            k_p2g_mom_chunks<kChunk><<<w.item_blocks, kChunkThreads, 0, st>>>(v, w.posm[cur], w.velid[cur],
-                                                                            w.aff[cur], w.cmf, mv, w.dens);
+            k_p2g_mom_chunks<kChunk><<<w.item_blocks, kChunkThreads, 0, st>>>(v, w.posm[cur], w.rows[cur], w.cmf, mv,
+                                                                            w.dens);
         w.launches++;
     }
     // the tail's ADVECT reads vel4 and its spawn pass the spawn bits that
@@ -2473,13 +2474,12 @@ static cudaError_t enqueue_substep(World& w, Scene* ds, const RefOut& ro, bool t
     {
         Phase ph(prof, MPM_PHASE_G2P);
         if (w.chunk == kChunkSmall)
-            k_g2p_chunks<kChunkSmall><<<w.item_blocks, kChunkThreads, 0, st>>>(v, w.posm[cur], w.velid[cur], w.vel4,
-                                                                             w.cmf, w.posm[nxt], w.velid[nxt],
-                                                                             w.aff[nxt], dv, ro);
+            k_g2p_chunks<kChunkSmall><<<w.item_blocks, kChunkThreads, 0, st>>>(v, w.posm[cur], w.pid[cur], w.vel4,
+                                                                             w.cmf, w.posm[nxt], w.rows[nxt],
+                                                                             w.pid[nxt], dv, ro);
         else
-            k_g2p_chunks<kChunk><<<w.item_blocks, kChunkThreads, 0, st>>>(v, w.posm[cur], w.velid[cur], w.vel4,
-                                                                        w.cmf, w.posm[nxt], w.velid[nxt],
-                                                                        w.aff[nxt], dv, ro);
+            k_g2p_chunks<kChunk><<<w.item_blocks, kChunkThreads, 0, st>>>(v, w.posm[cur], w.pid[cur], w.vel4, w.cmf,
+                                                                        w.posm[nxt], w.rows[nxt], w.pid[nxt], dv, ro);
         w.launches++;
     }
     w.cur = nxt;

@@ -193,8 +193,8 @@ struct World {
     uint32_t* tile_scene = nullptr;
     std::vector<uint32_t> h_tile_scene;
     float4* posm[2] = {nullptr, nullptr};   // (x, y, z, mass)
-    float4* velid[2] = {nullptr, nullptr};  // (vx, vy, vz, id bits)
-    float* aff[2] = {nullptr, nullptr};     // 9 planes of npos floats
+    float4* rows[2] = {nullptr, nullptr};   // 3 planes of npos: axis c's affine row and velocity (a_c0, a_c1, a_c2, v_c)
+    uint32_t* pid[2] = {nullptr, nullptr};  // particle ids
     float* dens = nullptr;
     uint32_t* cell_count = nullptr;
     uint32_t* cell_start = nullptr;
