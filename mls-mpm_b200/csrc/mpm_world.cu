@@ -102,18 +102,16 @@ WorldView World::view() const {
     WorldView v;
     v.npos = npos;
     v.ntiles = (uint32_t)tiles.high_water();
-    v.ngroups = (v.ntiles + 1023u) / 1024u;
-    if (v.ngroups == 0) v.ngroups = 1;
     v.chunk_cap = chunk_cap;
     v.chunk = chunk;
     v.scenes = scenes_dev(cur);
     v.tile_scene = tile_scene;
     v.cell_count = cell_count; v.cell_start = cell_start;
     v.key = key; v.rank = rank; v.perm = perm;
-    v.tile_flags = tile_flags; v.tile_occ = tile_occ; v.tile_cnt = tile_cnt;
-    v.tile_pstart = tile_pstart; v.tile_cstart = tile_cstart;
-    v.group_pstart = group_pstart; v.group_cstart = group_cstart;
-    v.chunk_info = chunk_info; v.chunk_last = chunk_last; v.chunk_hdr = chunk_hdr; v.chunk_geo = chunk_geo;
+    v.tile_flags = tile_flags; v.tile_cnt = tile_cnt; v.tile_base = tile_base;
+    v.par = (uint32_t)cur;
+    v.chunk_hdr = chunk_hdr[cur];
+    v.chunk_hdr_prev = chunk_hdr[cur ^ 1];
     v.tile_occ_list = tile_occ_list; v.tile_grid_list = tile_grid_list;
     v.ctrl = ctrl; v.dens = dens;
     v.health = health;
@@ -133,9 +131,12 @@ __device__ __forceinline__ uint32_t tile_of(const SceneDesc& sd, int32_t cx, int
            ((uint32_t)(cz / kTileZ) * sd.nty + (uint32_t)(cy / kTileY)) * sd.ntx + (uint32_t)(cx / kTileX);
 }
 
-// Mark a tile as holding particles for the next substep (bit 0).
-__device__ __forceinline__ void mark_occupied(const WorldView& v, uint32_t t) {
-    if ((v.tile_flags[t] & 1u) == 0u) atomicOr(&v.tile_flags[t], 1u);
+// Adds the active lanes' particles to their tiles' counts for the next binning:
+// one fire-and-forget add per distinct tile (neighbouring lanes mostly share one).
+__device__ __forceinline__ void count_in_tile(uint32_t* tile_cnt, uint32_t t) {
+    const unsigned act = __activemask();
+    const unsigned same = __match_any_sync(act, t);
+    if ((threadIdx.x & 31u) == (uint32_t)(__ffs(same) - 1)) atomicAdd(&tile_cnt[t], (uint32_t)__popc(same));
 }
 
 // Binning cell of a position (clamped into the scene's grid; binning only).
@@ -173,7 +174,7 @@ __global__ void k_import(WorldView v, uint32_t scene, uint32_t pos0, const float
     int32_t cx, cy, cz;
     bin_cell(sd, q.x, q.y, q.z, cx, cy, cz);
     v.key[p] = sd.cell_base + local_cell(sd, cx, cy, cz);
-    mark_occupied(v, tile_of(sd, cx, cy, cz));
+    count_in_tile(v.tile_cnt, tile_of(sd, cx, cy, cz));
 }
 
 // Drops a scene's particles: their positions become holes.
@@ -218,7 +219,6 @@ __global__ void k_export(WorldView v, const float4* __restrict__ posm, const flo
 // Sets the layout size after imports/removals done outside a substep.
 __global__ void k_set_total(Ctrl* ctrl, uint32_t total) {
     ctrl->total_pos = total;
-    ctrl->prev_total_pos = total;
 }
 
 // ---------------------------------------------------------------------------
@@ -242,17 +242,104 @@ __global__ void k_count_range(WorldView v, uint32_t p0, uint32_t p1) {
     }
 }
 
-// Occupied-tile list for the binning and the occupancy used by the scans.
-// tile_flags bits: 0 occupied (set by G2P / import), 1 stencil now (set by the
-// binning), 2 stencil last substep.
-__global__ void k_tiles_occ(WorldView v) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= v.ntiles) return;
-    const uint32_t occ = v.tile_flags[t] & 1u;
-    v.tile_occ[t] = occ;
-    if (occ) v.tile_occ_list[atomicAdd(&v.ctrl->n_occ, 1u)] = t;
+// tile_flags bits: 1 stencil now (set by the binning), 2 stencil last substep.
+
+// A tile's particles and chunks in one word, for scans of both.
+__device__ __forceinline__ uint64_t tile_load(const WorldView& v, uint32_t t) {
+    const uint32_t n = t < v.ntiles ? v.tile_cnt[t] : 0u;
+    return ((uint64_t)n << 32) | ((n + v.chunk - 1) / v.chunk);
 }
 
+// Scans one value a thread over a block of 1,024 tiles in index order: the
+// exclusive prefix of tile_load and the number of occupied tiles before the
+// thread's, and the block's sums.  buf holds 32 words of each, not in use by
+// the scan before.
+struct TileScan {
+    uint64_t load[32];
+    uint32_t occ[32];
+};
+__device__ __forceinline__ void tile_scan(uint64_t load, TileScan& buf, uint64_t& pre, uint32_t& before, uint64_t& sum,
+                                          uint32_t& n) {
+    const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+    const uint32_t w = __ballot_sync(0xffffffffu, load != 0);
+    uint64_t s = load;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint64_t a = __shfl_up_sync(0xffffffffu, s, d);
+        if (lane >= (uint32_t)d) s += a;
+    }
+    if (lane == 31) {
+        buf.load[wid] = s;
+        buf.occ[wid] = __popc(w);
+    }
+    __syncthreads();
+    uint64_t ws = buf.load[lane];
+    uint32_t wo = buf.occ[lane];
+    const uint64_t ws1 = ws;
+    const uint32_t wo1 = wo;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint64_t a = __shfl_up_sync(0xffffffffu, ws, d);
+        const uint32_t b = __shfl_up_sync(0xffffffffu, wo, d);
+        if (lane >= (uint32_t)d) {
+            ws += a;
+            wo += b;
+        }
+    }
+    pre = __shfl_sync(0xffffffffu, ws - ws1, wid) + s - load;
+    before = __shfl_sync(0xffffffffu, wo - wo1, wid) + __popc(w & ((1u << lane) - 1u));
+    sum = __shfl_sync(0xffffffffu, ws, 31);
+    n = __shfl_sync(0xffffffffu, wo, 31);
+}
+
+// The occupied tiles in index order with their first position and chunk, for
+// the binning of worlds of more than kScanTiles tiles: one block per 1,024
+// tiles, which adds up the tiles before its own by itself (no block waits for
+// another).
+__global__ void __launch_bounds__(1024) k_tiles_list(WorldView v) {
+    __shared__ TileScan buf[2];
+    __shared__ uint64_t part[32];
+    __shared__ uint32_t part_n[32];
+    const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+    uint64_t sum0 = 0;
+    uint32_t n0 = 0;
+    for (uint32_t t = threadIdx.x; t < blockIdx.x * 1024u; t += 1024u) {
+        const uint64_t l = tile_load(v, t);
+        sum0 += l;
+        n0 += l != 0;
+    }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) {
+        sum0 += __shfl_xor_sync(0xffffffffu, sum0, d);
+        n0 += __shfl_xor_sync(0xffffffffu, n0, d);
+    }
+    if (lane == 0) {
+        part[wid] = sum0;
+        part_n[wid] = n0;
+    }
+    __syncthreads();
+    sum0 = 0;
+    n0 = 0;
+    for (int k = 0; k < 32; ++k) {
+        sum0 += part[k];
+        n0 += part_n[k];
+    }
+    const uint32_t t = blockIdx.x * 1024u + threadIdx.x;
+    const uint64_t load = tile_load(v, t);
+    uint64_t pre, sum;
+    uint32_t before, n;
+    tile_scan(load, buf[0], pre, before, sum, n);
+    if (load != 0) {
+        pre += sum0;
+        v.tile_occ_list[n0 + before] = t;
+        v.tile_base[n0 + before] = make_uint2((uint32_t)(pre >> 32), (uint32_t)pre);
+    }
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+        v.ctrl->n_occ = n0 + n;
+        v.ctrl->cursor[v.par] = (uint32_t)((sum0 + sum) >> 32);
+        v.ctrl->chunks[v.par] = (uint32_t)(sum0 + sum);
+    }
+}
 
 __device__ __forceinline__ uint32_t block_exclusive_scan_1024(uint32_t x, uint32_t* ws, uint32_t& total) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -283,24 +370,122 @@ __device__ __forceinline__ uint32_t block_exclusive_scan_1024(uint32_t x, uint32
 }
 
 
-// One block per occupied tile, one thread per cell (local order x fastest,
-// then y, then z): exclusive scan of the cell counts inside the tile ->
-// cell_start (tile-local), tile total -> tile_cnt.  Also marks every tile the
-// particles' 3x3x3 stencils touch (bit 1).
-__device__ void tiles_fold(const WorldView& v, mpm_gen_params* gen);
+// ---------------------------------------------------------------------------
+// Chunks: the halo box of a chunk's cells
+// ---------------------------------------------------------------------------
+struct ChunkHdr {
+    uint32_t scene, first, end;
+    int32_t ox, oy, oz;      // scene-local cell at halo index 0
+    int32_t hx, hy, hz;      // halo dims
+};
 
-__global__ void __launch_bounds__(kTileCells) k_bin_cells(WorldView v, mpm_gen_params* gen, int fold) {
+// The box of the local cells [lo, hi] (x fastest, then y, then z) plus one
+// cell on every side.
+// The box of a chunk of tile (tx, ty, tz) of `scene` whose cells go from lo to hi.
+__device__ __forceinline__ void chunk_header_from(uint32_t scene, uint32_t tx, uint32_t ty, uint32_t tz, uint32_t lo,
+                                                  uint32_t hi, ChunkHdr& h) {
+    constexpr uint32_t kRow = kTileX, kSlab = kTileX * kTileY;
+    int32_t x0 = 0, x1 = kTileX - 1, y0 = 0, y1 = kTileY - 1;
+    const int32_t z0 = (int32_t)(lo / kSlab), z1 = (int32_t)(hi / kSlab);
+    if (z0 == z1) {
+        y0 = (int32_t)((lo / kRow) % kTileY);
+        y1 = (int32_t)((hi / kRow) % kTileY);
+        if (y0 == y1) {
+            x0 = (int32_t)(lo % kRow);
+            x1 = (int32_t)(hi % kRow);
+        }
+    }
+    h.scene = scene;
+    h.ox = (int32_t)tx * kTileX + x0 - 1;
+    h.oy = (int32_t)ty * kTileY + y0 - 1;
+    h.oz = (int32_t)tz * kTileZ + z0 - 1;
+    h.hx = x1 - x0 + 3;
+    h.hy = y1 - y0 + 3;
+    h.hz = z1 - z0 + 3;
+}
+
+// ChunkHdr packed in two 16-byte words (box dims below 256).
+__device__ __forceinline__ void pack_header(const ChunkHdr& h, uint4* dst) {
+    dst[0] = make_uint4(h.scene, h.first, h.end, (uint32_t)h.hx | ((uint32_t)h.hy << 8) | ((uint32_t)h.hz << 16));
+    dst[1] = make_uint4((uint32_t)h.ox, (uint32_t)h.oy, (uint32_t)h.oz, 0u);
+}
+__device__ __forceinline__ ChunkHdr unpack_header(const uint4 a, const uint4 b) {
+    ChunkHdr h;
+    h.scene = a.x;
+    h.first = a.y;
+    h.end = a.z;
+    h.hx = (int32_t)(a.w & 0xFFu);
+    h.hy = (int32_t)((a.w >> 8) & 0xFFu);
+    h.hz = (int32_t)((a.w >> 16) & 0xFFu);
+    h.ox = (int32_t)b.x;
+    h.oy = (int32_t)b.y;
+    h.oz = (int32_t)b.z;
+    return h;
+}
+
+
+// One block per occupied tile, one thread per cell (local order x fastest,
+// then y, then z): exclusive scan of the cell counts inside the tile; with the
+// tile's first position (tiles in index order), cell_start becomes the first
+// position of the cell's particles, the counts are cleared, and the tile's
+// chunk headers are written.  Also marks every tile the particles' 3x3x3
+// stencils touch (bit 1).  Block b takes the occupied tiles of number b,
+// b + gridDim, ...
+//
+// The tiles' first positions come from their particle counts, which G2P keeps:
+// in worlds of up to kScanTiles tiles every block scans the counts itself (one
+// load a thread for 1,024 tiles), in larger ones k_tiles_list does.  A scan of
+// the tile totals found by this kernel took two to five more launches (binning
+// 26 -> 15 us at 8,192 particles, 37 -> 22 us at 1M, 88 -> 72 us at 8M).
+// Handing positions out by one atomic cursor instead puts the tiles of the
+// blocks in flight in any order, which cost 10% of a substep at 8M (the render
+// mirrors' writes by id and the grid's halos then miss L2).
+constexpr uint32_t kScanTiles = 16384;
+constexpr uint32_t kBinMine = 256;   // tiles of one block in such a world
+__global__ void __launch_bounds__(kTileCells) k_bin_cells(WorldView v) {
     __shared__ uint32_t ws[33];
     __shared__ uint32_t dirs;
-    const uint32_t nocc = v.ctrl->n_occ;
-    for (uint32_t ti = blockIdx.x; ti < nocc; ti += gridDim.x) {
-        const uint32_t t = v.tile_occ_list[ti];
+    __shared__ uint32_t mine[kBinMine];
+    __shared__ uint2 mine_base[kBinMine];
+    __shared__ TileScan buf[2];
+    const bool listed = v.ntiles > kScanTiles;
+    uint32_t nocc = 0;
+    if (listed) {
+        nocc = v.ctrl->n_occ;
+    } else {
+        uint64_t all = 0;
+        for (uint32_t t0 = 0, it = 0; t0 < v.ntiles; t0 += kTileCells, ++it) {
+            const uint32_t t = t0 + threadIdx.x;
+            const uint64_t load = tile_load(v, t);
+            uint64_t pre, sum;
+            uint32_t before, n;
+            tile_scan(load, buf[it & 1u], pre, before, sum, n);   // (one barrier a scan: the buffers alternate)
+            const uint32_t i = nocc + before;
+            if (load != 0 && i % gridDim.x == blockIdx.x) {
+                pre += all;
+                mine[i / gridDim.x] = t;
+                mine_base[i / gridDim.x] = make_uint2((uint32_t)(pre >> 32), (uint32_t)pre);
+            }
+            nocc += n;
+            all += sum;
+        }
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            v.ctrl->cursor[v.par] = (uint32_t)(all >> 32);
+            v.ctrl->chunks[v.par] = (uint32_t)all;
+        }
+        __syncthreads();
+    }
+    for (uint32_t ti = blockIdx.x, k = 0; ti < nocc; ti += gridDim.x, ++k) {
+        const uint32_t t = listed ? v.tile_occ_list[ti] : mine[k];
+        const uint2 base = listed ? v.tile_base[ti] : mine_base[k];
+        const uint32_t base_p = base.x, base_c = base.y;
         const uint32_t scene = v.tile_scene[t];
+        if (scene == kHole) continue;   // block-uniform
         const SceneDesc& sd = v.scenes[scene];
         const uint32_t lt = t - sd.tile_base;
         const uint32_t tx = lt % sd.ntx, ty = (lt / sd.ntx) % sd.nty, tz = lt / (sd.ntx * sd.nty);
-        const uint32_t lx = threadIdx.x % kTileX, ly = (threadIdx.x / kTileX) % kTileY,
-                       lz = threadIdx.x / (kTileX * kTileY);
+        const uint32_t lid = threadIdx.x;
+        const uint32_t lx = lid % kTileX, ly = (lid / kTileX) % kTileY, lz = lid / (kTileX * kTileY);
         const uint32_t x = tx * kTileX + lx, y = ty * kTileY + ly, z = tz * kTileZ + lz;
         const bool inside = x < sd.X && y < sd.Y && z < sd.Z;
         const uint32_t c = inside ? sd.cell_base + local_cell(sd, x, y, z) : 0u;
@@ -321,9 +506,8 @@ __global__ void __launch_bounds__(kTileCells) k_bin_cells(WorldView v, mpm_gen_p
         const uint32_t wm = __reduce_or_sync(0xffffffffu, m);
         if ((threadIdx.x & 31) == 0 && wm) atomicOr(&dirs, wm);
         uint32_t total;
-        const uint32_t local = block_exclusive_scan_1024(cnt, ws, total);   // also orders the dirs updates
-        if (cnt) v.cell_start[c] = local;
-        if (threadIdx.x == 0) v.tile_cnt[t] = total;
+        const uint32_t a = block_exclusive_scan_1024(cnt, ws, total);   // also orders the dirs updates
+        const uint32_t C = v.chunk, nch = (total + C - 1) / C;   // total: the tile's count, as G2P kept it
         if (threadIdx.x < 27 && ((dirs >> threadIdx.x) & 1u)) {
             const int ox = (int)(threadIdx.x % 3) - 1, oy = (int)((threadIdx.x / 3) % 3) - 1,
                       oz = (int)(threadIdx.x / 9) - 1;
@@ -333,29 +517,37 @@ __global__ void __launch_bounds__(kTileCells) k_bin_cells(WorldView v, mpm_gen_p
                 if ((v.tile_flags[nt] & 2u) == 0u) atomicOr(&v.tile_flags[nt], 2u);
             }
         }
+        if (cnt) {
+            v.cell_start[c] = base_p + a;
+            v.cell_count[c] = 0u;
+            // the first and the last local cell of every chunk that starts or ends
+            // in this cell, left in the chunk's second header word
+            for (uint32_t j = a / C; j <= (a + cnt - 1) / C && base_c + j < v.chunk_cap; ++j) {
+                uint32_t* w = reinterpret_cast<uint32_t*>(v.chunk_hdr + 2ull * (base_c + j) + 1);
+                if (j * C >= a) w[0] = lid;
+                if (min(j * C + C, total) <= a + cnt) w[1] = lid;
+            }
+        }
+        __syncthreads();
+        for (uint32_t j = threadIdx.x; j < nch && base_c + j < v.chunk_cap; j += kTileCells) {
+            uint4* out = v.chunk_hdr + 2ull * (base_c + j);
+            const uint4 cells = out[1];
+            ChunkHdr h;
+            chunk_header_from(scene, tx, ty, tz, cells.x, cells.y, h);
+            h.first = base_p + j * C;
+            h.end = base_p + min(j * C + C, total);
+            pack_header(h, out);
+        }
         __syncthreads();
     }
-    if (!fold) return;
-    // the last block to finish runs the per-tile passes (block-uniform test)
-    __shared__ bool last;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        last = atomicAdd(&v.ctrl->bins_done, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    tiles_fold(v, gen);
 }
 
 // Grid-tile list (stencil tiles of this substep or the last one, plus the
 // hand boxes); shifts the flags for the next substep.
-// (The flags are read past L1: in the folded form other blocks of the same
-// kernel have just set their bit 1.)
 __device__ __forceinline__ void tile_grid_entry(const WorldView& v, uint32_t t) {
     const uint32_t scene = v.tile_scene[t];
-    const uint32_t f = __ldcg(v.tile_flags + t);
+    const uint32_t f = v.tile_flags[t];
+    v.tile_cnt[t] = 0u;   // (the binning has read it; this substep's G2P counts anew)
     if (scene == kHole) {
         if (f) v.tile_flags[t] = 0u;
         return;
@@ -369,151 +561,20 @@ __device__ __forceinline__ void tile_grid_entry(const WorldView& v, uint32_t t) 
         hand = x0 <= sd.hand_box[3] && x0 + kTileX - 1 >= sd.hand_box[0] && y0 <= sd.hand_box[4] &&
                y0 + kTileY - 1 >= sd.hand_box[1] && z0 <= sd.hand_box[5] && z0 + kTileZ - 1 >= sd.hand_box[2];
     }
-    const bool now = (f & 2u) != 0 || hand || (v.tile_occ[t] != 0u);
+    const bool now = (f & 2u) != 0 || hand;
     const bool prev = (f & 4u) != 0;
     if (now || prev) v.tile_grid_list[atomicAdd(&v.ctrl->n_grid, 1u)] = t;
     if (f != (now ? 4u : 0u)) v.tile_flags[t] = now ? 4u : 0u;
 }
 
-__global__ void k_tiles_grid(WorldView v) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < v.ntiles) tile_grid_entry(v, t);
-}
-
-
-// Two-level exclusive scan over all tiles in index order of the particle
-// counts and the chunk counts of the occupied tiles.  Level 1, one block per
-// group of 1024 tiles: prefixes inside the group, group totals.
-__global__ void __launch_bounds__(1024) k_tile_scan_local(WorldView v) {
-    __shared__ uint32_t ws[33];
-    const uint32_t g = blockIdx.x;
-    const uint32_t t = g * 1024u + threadIdx.x;
-    const uint32_t np = (t < v.ntiles && v.tile_occ[t]) ? v.tile_cnt[t] : 0u;
-    const uint32_t nc = (np + v.chunk - 1) / v.chunk;
-    uint32_t tp, tc;
-    const uint32_t rp = block_exclusive_scan_1024(np, ws, tp);
-    const uint32_t rc = block_exclusive_scan_1024(nc, ws, tc);
-    if (t < v.ntiles) {
-        v.tile_pstart[t] = rp;
-        v.tile_cstart[t] = rc;
-    }
-    if (threadIdx.x == 0) {
-        v.group_pstart[g] = tp;
-        v.group_cstart[g] = tc;
-    }
-}
-
-// Level 2, one block: exclusive scan of the group totals; the layout size and
-// chunk count go to ctrl.  Also advances the diffuse seed (diffuse-gpu.js:149).
-__global__ void __launch_bounds__(1024) k_tile_scan_top(WorldView v, mpm_gen_params* gen) {
-    __shared__ uint32_t ws[33];
-    uint32_t cp = 0, cc = 0;
-    for (uint32_t g0 = 0; g0 < v.ngroups; g0 += 1024) {
-        const uint32_t g = g0 + threadIdx.x;
-        const uint32_t xp = g < v.ngroups ? v.group_pstart[g] : 0u;
-        const uint32_t xc = g < v.ngroups ? v.group_cstart[g] : 0u;
-        uint32_t tp, tc;
-        const uint32_t rp = block_exclusive_scan_1024(xp, ws, tp);
-        const uint32_t rc = block_exclusive_scan_1024(xc, ws, tc);
-        if (g < v.ngroups) {
-            v.group_pstart[g] = cp + rp;
-            v.group_cstart[g] = cc + rc;
-        }
-        cp += tp;
-        cc += tc;
-    }
-    if (threadIdx.x == 0) {
-        v.ctrl->prev_total_pos = v.ctrl->total_pos;
-        v.ctrl->total_pos = min(cp, v.npos);
-        v.ctrl->total_chunks = min(cc, v.chunk_cap);
-        if (gen) gen->seed = gen->seed + 1u;
-    }
-}
-
-// Tiles of a world small enough for one block to finish the binning's
-// per-tile passes: the last k_bin_cells block to finish builds the grid-tile
-// list and scans the tile counts itself instead of three more launches.
-constexpr uint32_t kFoldTiles = 4096;
-
-// The grid-tile list and the exclusive scans of the particle and chunk counts
-// over all tiles (tile_pstart/tile_cstart global, group offsets 0), the layout
-// totals and the diffuse seed bump: the work of k_tiles_grid,
-// k_tile_scan_local and k_tile_scan_top, by one 1024-thread block.
-__device__ void tiles_fold(const WorldView& v, mpm_gen_params* gen) {
-    __shared__ uint32_t ws[33];
-    for (uint32_t t = threadIdx.x; t < v.ntiles; t += blockDim.x) tile_grid_entry(v, t);
-    uint32_t cp = 0, cc = 0;
-    for (uint32_t t0 = 0; t0 < v.ntiles; t0 += 1024) {
-        const uint32_t t = t0 + threadIdx.x;
-        // tile counts written by the other blocks of k_bin_cells: read past L1
-        const uint32_t np = (t < v.ntiles && v.tile_occ[t]) ? __ldcg(v.tile_cnt + t) : 0u;
-        const uint32_t nc = (np + v.chunk - 1) / v.chunk;
-        uint32_t tp, tc;
-        const uint32_t rp = block_exclusive_scan_1024(np, ws, tp);
-        const uint32_t rc = block_exclusive_scan_1024(nc, ws, tc);
-        if (t < v.ntiles) {
-            v.tile_pstart[t] = cp + rp;
-            v.tile_cstart[t] = cc + rc;
-        }
-        cp += tp;
-        cc += tc;
-    }
-    for (uint32_t g = threadIdx.x; g < v.ngroups; g += blockDim.x) {
-        v.group_pstart[g] = 0u;
-        v.group_cstart[g] = 0u;
-    }
-    if (threadIdx.x == 0) {
-        v.ctrl->prev_total_pos = v.ctrl->total_pos;
-        v.ctrl->total_pos = min(cp, v.npos);
-        v.ctrl->total_chunks = min(cc, v.chunk_cap);
-        if (gen) gen->seed = gen->seed + 1u;
-    }
-}
-
-// One block per occupied tile, one thread per cell: cell_start becomes the
-// global first position, the counts are cleared, and the tile's chunks are
-// written: (tile, first position, end position, first local cell) and the
-// last local cell, each by the thread whose cell holds that particle.
-__global__ void __launch_bounds__(kTileCells) k_tile_finish(WorldView v) {
-    const uint32_t nocc = v.ctrl->n_occ;
-    for (uint32_t ti = blockIdx.x; ti < nocc; ti += gridDim.x) {
-        const uint32_t t = v.tile_occ_list[ti];
-        const uint32_t scene = v.tile_scene[t];
-        const SceneDesc& sd = v.scenes[scene];
-        const uint32_t lt = t - sd.tile_base;
-        const uint32_t tx = lt % sd.ntx, ty = (lt / sd.ntx) % sd.nty, tz = lt / (sd.ntx * sd.nty);
-        const uint32_t lid = threadIdx.x;
-        const uint32_t x = tx * kTileX + lid % kTileX, y = ty * kTileY + (lid / kTileX) % kTileY,
-                       z = tz * kTileZ + lid / (kTileX * kTileY);
-        if (x >= sd.X || y >= sd.Y || z >= sd.Z) continue;
-        const uint32_t c = sd.cell_base + local_cell(sd, x, y, z);
-        const uint32_t cnt = v.cell_count[c];
-        if (cnt == 0) continue;
-        const uint32_t base_p = v.tile_pstart[t] + v.group_pstart[t >> 10];
-        const uint32_t base_c = v.tile_cstart[t] + v.group_cstart[t >> 10];
-        const uint32_t total = v.tile_cnt[t];
-        const uint32_t a = v.cell_start[c];
-        v.cell_start[c] = base_p + a;
-        v.cell_count[c] = 0u;
-        const uint32_t C = v.chunk;
-        for (uint32_t j = a / C; j <= (a + cnt - 1) / C; ++j) {
-            const uint32_t ci = base_c + j;
-            if (ci >= v.chunk_cap) break;
-            const uint32_t f = j * C;
-            const uint32_t e = min(f + C, total);
-            if (f >= a) {
-                v.chunk_info[ci] = make_uint4(t, base_p + f, base_p + e, lid);
-                v.chunk_geo[ci] = make_uint4(scene, tx, ty, tz);
-            }
-            if (e - 1 < a + cnt) v.chunk_last[ci] = lid;
-        }
-    }
-}
-
-// perm[new position] = previous position for every particle.
-__global__ void k_scatter(WorldView v) {
-    const uint32_t total = v.ctrl->prev_total_pos;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+// perm[new position] = previous position for every particle, and the
+// grid-tile list.  Also advances the diffuse seed (diffuse-gpu.js:149).
+__global__ void k_scatter(WorldView v, mpm_gen_params* gen) {
+    const uint32_t total = v.ctrl->total_pos;   // (of the previous layout: DECODE_MASS sets this one's)
+    const uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+    if (i0 == 0 && gen) gen->seed = gen->seed + 1u;
+    for (uint32_t t = i0; t < v.ntiles; t += stride) tile_grid_entry(v, t);
+    for (uint32_t i = i0; i < total; i += stride) {
         const uint32_t c = v.key[i];
         if (c == kHole) continue;
         const uint32_t pos = v.cell_start[c] + v.rank[i];
@@ -590,8 +651,13 @@ __device__ __forceinline__ float2 sadd(float2 a, float2 b) { return make_float2(
 
 
 // ---------------------------------------------------------------------------
-// Chunks: the halo box of a chunk's cells in shared memory
+// Chunks in shared memory
 // ---------------------------------------------------------------------------
+// Chunks of the layout of parity p.
+__device__ __forceinline__ uint32_t chunk_count(const WorldView& v, uint32_t p) {
+    return min(v.ctrl->chunks[p], v.chunk_cap);
+}
+
 // Lane order of the P2G chunk kernels: lane l of warp w has offset 8*l + w
 // (8 warps per block), which chunk_slot scales to a particle of the chunk, so
 // neighbouring lanes sit in different cells and the lanes of one shared
@@ -620,42 +686,6 @@ __device__ __forceinline__ uint32_t chunk_slot(int r) {
 #endif
 }
 
-struct ChunkHdr {
-    uint32_t scene, first, end;
-    int32_t ox, oy, oz;      // scene-local cell at halo index 0
-    int32_t hx, hy, hz;      // halo dims
-};
-
-// The box of the local cells [lo, hi] (x fastest, then y, then z) plus one
-// cell on every side.
-// The chunk's header from its three independent words: chunk_info (tile,
-// first, end, first local cell), chunk_last (last local cell) and chunk_geo
-// (scene, tile coordinates).
-__device__ __forceinline__ void chunk_header_from(const uint4 ci, uint32_t hi, const uint4 geo, ChunkHdr& h) {
-    const uint32_t lo = ci.w;
-    const int32_t tx = (int32_t)geo.y, ty = (int32_t)geo.z, tz = (int32_t)geo.w;
-    constexpr uint32_t kRow = kTileX, kSlab = kTileX * kTileY;
-    int32_t x0 = 0, x1 = kTileX - 1, y0 = 0, y1 = kTileY - 1;
-    const int32_t z0 = (int32_t)(lo / kSlab), z1 = (int32_t)(hi / kSlab);
-    if (z0 == z1) {
-        y0 = (int32_t)((lo / kRow) % kTileY);
-        y1 = (int32_t)((hi / kRow) % kTileY);
-        if (y0 == y1) {
-            x0 = (int32_t)(lo % kRow);
-            x1 = (int32_t)(hi % kRow);
-        }
-    }
-    h.scene = geo.x;
-    h.first = ci.y;
-    h.end = ci.z;
-    h.ox = tx * kTileX + x0 - 1;
-    h.oy = ty * kTileY + y0 - 1;
-    h.oz = tz * kTileZ + z0 - 1;
-    h.hx = x1 - x0 + 3;
-    h.hy = y1 - y0 + 3;
-    h.hz = z1 - z0 + 3;
-}
-
 // Asynchronous 16-byte global -> shared copy (cp.async); src_bytes 0 writes
 // zeros.  cp_async_wait waits for all of this thread's copies.
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem, uint32_t src_bytes) {
@@ -669,25 +699,6 @@ __device__ __forceinline__ void cp_async4z(void* smem, const void* gmem, uint32_
 }
 __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
-}
-
-// ChunkHdr packed in two 16-byte words (box dims below 256).
-__device__ __forceinline__ void pack_header(const ChunkHdr& h, uint4* dst) {
-    dst[0] = make_uint4(h.scene, h.first, h.end, (uint32_t)h.hx | ((uint32_t)h.hy << 8) | ((uint32_t)h.hz << 16));
-    dst[1] = make_uint4((uint32_t)h.ox, (uint32_t)h.oy, (uint32_t)h.oz, 0u);
-}
-__device__ __forceinline__ ChunkHdr unpack_header(const uint4 a, const uint4 b) {
-    ChunkHdr h;
-    h.scene = a.x;
-    h.first = a.y;
-    h.end = a.z;
-    h.hx = (int32_t)(a.w & 0xFFu);
-    h.hy = (int32_t)((a.w >> 8) & 0xFFu);
-    h.hz = (int32_t)((a.w >> 16) & 0xFFu);
-    h.ox = (int32_t)b.x;
-    h.oy = (int32_t)b.y;
-    h.oz = (int32_t)b.z;
-    return h;
 }
 
 // Each block of the chunk kernels keeps its chunk's scene descriptor in
@@ -795,20 +806,17 @@ __global__ void __launch_bounds__(kChunkThreads) k_p2g_mass_chunks(WorldView v, 
                                                                    int32_t* __restrict__ cm) {
     constexpr int kPer = kC / kChunkThreads;
     __shared__ int32_t acc[kHaloCells];
-    const uint32_t nch = v.ctrl->total_chunks;
+    const uint32_t nch = chunk_count(v, v.par);
     __shared__ ChunkHdr hs;
+    __shared__ uint4 nhs[2];                         // the next chunk's header words
     // scene descriptors of this chunk and the next (thread 0 copies the next
     // one while this chunk runs)
     __shared__ SceneDesc ssd[2];
     int sb = 0;                                      // ssd[sb]: this chunk's scene
     uint32_t ss_nxt = kHole;                         // thread 0: scene held in ssd[sb ^ 1]
-    // thread 0: the next chunk's header words, loaded while this chunk runs
-    uint4 nci = make_uint4(0u, 0u, 0u, 0u), ngeo = nci;
-    uint32_t nlast = 0;
     if (threadIdx.x == 0 && blockIdx.x < nch) {
-        const uint4 g0 = v.chunk_geo[blockIdx.x];
-        chunk_header_from(v.chunk_info[blockIdx.x], v.chunk_last[blockIdx.x], g0, hs);
-        copy_scene_async_one(v, g0.x, ssd[0]);
+        hs = unpack_header(v.chunk_hdr[2ull * blockIdx.x], v.chunk_hdr[2ull * blockIdx.x + 1]);
+        copy_scene_async_one(v, hs.scene, ssd[0]);
         cp_async_wait();
     }
     // the accumulators start at zero and every flush zeroes what it read
@@ -817,13 +825,9 @@ __global__ void __launch_bounds__(kChunkThreads) k_p2g_mass_chunks(WorldView v, 
     for (uint32_t ch = blockIdx.x; ch < nch; ch += gridDim.x) {
         const ChunkHdr h = hs;
         const uint32_t nxt = ch + gridDim.x;
-        if (threadIdx.x == 0) {
-            pack_header(h, v.chunk_hdr + 2ull * ch);   // for P2G_MOM and G2P
-            if (nxt < nch) {
-                nci = v.chunk_info[nxt];
-                nlast = v.chunk_last[nxt];
-                ngeo = v.chunk_geo[nxt];
-            }
+        if (threadIdx.x == 0 && nxt < nch) {
+            cp_async16(&nhs[0], v.chunk_hdr + 2ull * nxt, 16u);
+            cp_async16(&nhs[1], v.chunk_hdr + 2ull * nxt + 1, 16u);
         }
         // this thread's particles, all loads issued before the first is used
         float4 q[kPer];
@@ -871,10 +875,11 @@ __global__ void __launch_bounds__(kChunkThreads) k_p2g_mass_chunks(WorldView v, 
         __syncthreads();
         // every thread holds this chunk's header: the next one can replace it
         if (threadIdx.x == 0 && nxt < nch) {
-            chunk_header_from(nci, nlast, ngeo, hs);
-            if (ngeo.x != ss_nxt) {
-                copy_scene_async_one(v, ngeo.x, ssd[sb ^ 1]);
-                ss_nxt = ngeo.x;
+            cp_async_wait();
+            hs = unpack_header(nhs[0], nhs[1]);
+            if (hs.scene != ss_nxt) {
+                copy_scene_async_one(v, hs.scene, ssd[sb ^ 1]);
+                ss_nxt = hs.scene;
             }
         }
         int32_t* scm = cm + sd.cell_base;
@@ -914,6 +919,8 @@ __device__ __forceinline__ const SceneDesc* tile_cell(const WorldView& v, uint32
 
 __global__ void __launch_bounds__(256) k_decode_tiles(WorldView v, const int32_t* __restrict__ cm,
                                                       float* __restrict__ cmf) {
+    // the binning is done: the layout's size for the passes between substeps
+    if (blockIdx.x == 0 && threadIdx.x == 0) v.ctrl->total_pos = min(v.ctrl->cursor[v.par], v.npos);
     const uint32_t total = v.ctrl->n_grid * kTileCells;
     for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x) {
         uint32_t c;
@@ -1398,7 +1405,7 @@ __global__ void __launch_bounds__(kChunkThreads, MPM_MOM_MINB) k_p2g_mom_chunks(
     // the scene descriptors of the current chunk and of the next one, which is
     // copied while the current chunk runs (no wait when the scene changes)
     __shared__ SceneDesc ssd[2];
-    const uint32_t nch = v.ctrl->total_chunks;
+    const uint32_t nch = chunk_count(v, v.par);
     const uint32_t G = gridDim.x;
     if (blockIdx.x >= nch) return;   // block-uniform
     const size_t plane = v.npos;
@@ -1691,7 +1698,7 @@ struct G2POut {
     uint32_t* key;
     uint32_t* rank;
     uint32_t* cell_count;
-    uint32_t* tile_flags;
+    uint32_t* tile_cnt;
     const float* dens;
     const float* cmf;                    // scene's decoded cell masses
     const mpm_gen_params* gen;           // null: no spawning for this scene
@@ -1753,14 +1760,7 @@ __device__ __forceinline__ uint32_t g2p_store(const G2POut& o, const SceneDesc& 
     o.key[p] = key;
     // the rank within the cell for the next substep's binning (k_count's work)
     const uint32_t rank = atomicAdd(&o.cell_count[key], 1u);
-    // occupied-tile mark: one fire-and-forget OR per distinct tile of the
-    // active lanes (consecutive positions mostly share one tile)
-    {
-        const uint32_t t = tile_of(sd, cx, cy, cz);
-        const unsigned act = __activemask();
-        const unsigned same = __match_any_sync(act, t);
-        if ((threadIdx.x & 31u) == (uint32_t)(__ffs(same) - 1)) atomicOr(&o.tile_flags[t], 1u);
-    }
+    count_in_tile(o.tile_cnt, tile_of(sd, cx, cy, cz));
     if (o.gen) {
         const uint32_t id = gid - sd.id_base;
         // spawn_record's first test (shaders.js:806), checked inline
@@ -1838,7 +1838,7 @@ __global__ void __launch_bounds__(kChunkThreads, MPM_G2P_MINB) k_g2p_chunks(Worl
     constexpr int kPer = kC / kChunkThreads;
     __shared__ float4 vh[kHaloCells];   // staged grid velocities (x, y, z, 0)
     __shared__ uint4 nhs[2];              // the next chunk's header words
-    const uint32_t nch = v.ctrl->total_chunks;
+    const uint32_t nch = chunk_count(v, v.par);
     const size_t plane = v.npos;
     __shared__ ChunkHdr hs;
     // scene descriptors of this chunk and the next (thread 0 copies the next
@@ -1853,11 +1853,7 @@ __global__ void __launch_bounds__(kChunkThreads, MPM_G2P_MINB) k_g2p_chunks(Worl
     const float ke_threshold = dv.enabled ? dv.gen->ke_threshold : 0.0f;
     // the per-substep counters of the binning and the grid passes are read
     // no more in this substep: clear them for the next one
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        v.ctrl->n_occ = 0u;
-        v.ctrl->n_grid = 0u;
-        v.ctrl->bins_done = 0u;
-    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) v.ctrl->n_grid = 0u;
     // chunk headers: the next one's words are copied while this chunk runs
     if (threadIdx.x == 0 && blockIdx.x < nch) {
         hs = unpack_header(v.chunk_hdr[2ull * blockIdx.x], v.chunk_hdr[2ull * blockIdx.x + 1]);
@@ -1905,7 +1901,7 @@ __global__ void __launch_bounds__(kChunkThreads, MPM_G2P_MINB) k_g2p_chunks(Worl
         }
         const bool spawn_scene = dv.enabled && h.scene == dv.scene;
         const bool mirror = ro.enabled && h.scene == ro.scene;
-        const G2POut out{posm_out, rows_out, ids_out, plane, v.key, v.rank, v.cell_count, v.tile_flags, v.dens,
+        const G2POut out{posm_out, rows_out, ids_out, plane, v.key, v.rank, v.cell_count, v.tile_cnt, v.dens,
                          cmf + sd.cell_base, spawn_scene ? dv.gen : nullptr, bubble_min, pressure_threshold,
                          ke_threshold, dv.staging, dv.spawn_bits, dv.group_counts};
 #pragma unroll 1
@@ -1990,7 +1986,6 @@ static void world_plan(World& w, uint32_t particle_cap, uint64_t cell_cap, uint3
 // release and the footprint).
 template <class F> static void world_arrays(World& w, F&& f) {
     const size_t P = w.npos, C = w.cell_cap ? w.cell_cap : 1, T = w.tile_cap;
-    const size_t NG = (T + 1023) / 1024 + 1;
     for (int b = 0; b < 2; ++b) {
         f(w.posm[b], P * 16);
         f(w.rows[b], P * 48);
@@ -2004,16 +1999,10 @@ template <class F> static void world_arrays(World& w, F&& f) {
     f(w.rank, P * 4);
     f(w.perm, P * 4);
     f(w.tile_flags, T * 4);
-    f(w.tile_occ, T * 4);
     f(w.tile_cnt, T * 4);
-    f(w.tile_pstart, T * 4);
-    f(w.tile_cstart, T * 4);
-    f(w.group_pstart, NG * 4);
-    f(w.group_cstart, NG * 4);
-    f(w.chunk_info, (size_t)w.chunk_cap * 16);
-    f(w.chunk_last, (size_t)w.chunk_cap * 4);
-    f(w.chunk_hdr, (size_t)w.chunk_cap * 32);
-    f(w.chunk_geo, (size_t)w.chunk_cap * 16);
+    f(w.tile_base, T * 8);
+    f(w.chunk_hdr[0], (size_t)w.chunk_cap * 32);
+    f(w.chunk_hdr[1], (size_t)w.chunk_cap * 32);
     f(w.tile_occ_list, T * 4);
     f(w.tile_grid_list, T * 4);
     f(w.tile_scene, T * 4);
@@ -2050,7 +2039,7 @@ cudaError_t world_alloc(World& w, int device, cudaStream_t stream, uint32_t part
     w.sms = (uint32_t)sms;
     w.item_blocks = (uint32_t)sms * 4;
     w.grid_blocks = (uint32_t)sms * 8;
-    w.bin_blocks = (uint32_t)sms * 2;
+    w.bin_blocks = std::max((uint32_t)sms * 2, kScanTiles / kBinMine);
     w.pos_blocks = std::min<uint32_t>(cdiv(w.npos, 256), (uint32_t)sms * 16);
     const size_t P = w.npos, C = cell_cap ? cell_cap : 1, T = w.tile_cap;
     cudaError_t e = cudaSuccess;
@@ -2077,7 +2066,7 @@ cudaError_t world_alloc(World& w, int device, cudaStream_t stream, uint32_t part
     if (e == cudaSuccess) e = cudaMemsetAsync(w.vel4, 0, C * 16, stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(w.cell_count, 0, (C + 1) * 4, stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(w.tile_flags, 0, T * 4, stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(w.tile_occ, 0, T * 4, stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(w.tile_cnt, 0, T * 4, stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(w.dens, 0, P * 4, stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(w.ctrl, 0, sizeof(Ctrl), stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(w.health, 0, (size_t)(scene_cap ? scene_cap : 1) * 4, stream);
@@ -2333,6 +2322,7 @@ cudaError_t world_remove_scene(World& w, int slot) {
     if (e == cudaSuccess) e = cudaMemsetAsync(w.mvf + 3ull * r.cell_base, 0, (size_t)r.G * 12, w.stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(w.vel4 + r.cell_base, 0, (size_t)r.G * 16, w.stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(w.tile_flags + r.tile_base, 0, (size_t)r.ntiles * 4, w.stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(w.tile_cnt + r.tile_base, 0, (size_t)r.ntiles * 4, w.stream);
     // the counts G2P left in the scene's cells: the other scenes' counts and
     // ranks stay valid, so no recount is needed
     if (e == cudaSuccess) e = cudaMemsetAsync(w.cell_count + r.cell_base, 0, (size_t)r.G * 4, w.stream);
@@ -2384,7 +2374,6 @@ static cudaError_t enqueue_substep(World& w, Scene* ds, const RefOut& ro, bool t
     int32_t* cm_n = w.grid_i32[w.gbuf ^ 1];
     int32_t* mv_n = cm_n + w.cell_cap;
     const uint32_t nposb = w.pos_blocks;
-    const uint32_t ntb = cdiv(v.ntiles ? v.ntiles : 1, 256);
     DiffuseView dv{};
     mpm_gen_params* gen_dev = nullptr;
     if (ds && ds->diffuse.enabled) {
@@ -2419,21 +2408,13 @@ static cudaError_t enqueue_substep(World& w, Scene* ds, const RefOut& ro, bool t
             k_count<<<nposb, 256, 0, st>>>(v);
             w.launches++;
         }
-        k_tiles_occ<<<ntb, 256, 0, st>>>(v);
-        if (v.ntiles <= kFoldTiles) {
-            // the last binning block builds the grid list and scans the tiles
-            k_bin_cells<<<w.bin_blocks, kTileCells, 0, st>>>(v, gen_dev, 1);
-            w.launches += 1;
-        } else {
-            k_bin_cells<<<w.bin_blocks, kTileCells, 0, st>>>(v, gen_dev, 0);
-            k_tiles_grid<<<ntb, 256, 0, st>>>(v);
-            k_tile_scan_local<<<v.ngroups, 1024, 0, st>>>(v);
-            k_tile_scan_top<<<1, 1024, 0, st>>>(v, gen_dev);
-            w.launches += 4;
+        if (v.ntiles > kScanTiles) {
+            k_tiles_list<<<cdiv(v.ntiles, 1024), 1024, 0, st>>>(v);
+            w.launches++;
         }
-        k_tile_finish<<<w.bin_blocks, kTileCells, 0, st>>>(v);
-        k_scatter<<<nposb, 256, 0, st>>>(v);
-        w.launches += 3;
+        k_bin_cells<<<w.bin_blocks, kTileCells, 0, st>>>(v);
+        k_scatter<<<nposb, 256, 0, st>>>(v, gen_dev);
+        w.launches += 2;
     }
     {
         Phase ph(prof, MPM_PHASE_P2G_MASS);
@@ -2491,7 +2472,7 @@ static cudaError_t enqueue_substep(World& w, Scene* ds, const RefOut& ro, bool t
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     if (dv.enabled) {
-        ds->diffuse.seed += 1u;   // mirrors the device-side bump in k_tile_scan_top
+        ds->diffuse.seed += 1u;   // mirrors the device-side bump in k_scatter
         const SceneDesc* sd_dev = w.scenes_dev(cur) + dv.scene;
         if (defer) {
             // this substep's uniforms for its deferred tail (the scene table may

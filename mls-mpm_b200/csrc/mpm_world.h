@@ -59,44 +59,36 @@ struct alignas(16) SceneDesc {
 };
 static_assert(sizeof(SceneDesc) == 576, "bench.py SCENE_DESC_BYTES counts this block per uniform upload");
 
-// Small device-side control block.  The first kCtrlZeroBytes (per-substep
-// counters) start at zero and are cleared again by G2P, which runs after
-// their last use in the substep.
+// Small device-side control block; starts at zero.
 struct Ctrl {
-    uint32_t n_occ, n_grid, bins_done, pad1;   // bins_done: k_bin_cells blocks finished
-    // persistent
-    uint32_t total_chunks;      // chunks of the current layout
-    uint32_t total_pos;         // positions of the current layout
-    uint32_t prev_total_pos;    // positions of the previous layout (read through perm)
-    uint32_t pad2;
+    uint32_t n_occ;             // occupied tiles listed for the binning (worlds of many tiles)
+    uint32_t n_grid;            // grid tiles of this substep (cleared by G2P, after their last use)
+    uint32_t total_pos;         // positions of the layout, holes of removed scenes included
+    uint32_t pad;
+    // by substep parity, written by the binning
+    uint32_t cursor[2];         // positions of the layout
+    uint32_t chunks[2];         // chunks of the layout
 };
-constexpr size_t kCtrlZeroBytes = 16;
 
 // Everything the device kernels need (passed by value).
 struct WorldView {
     uint32_t npos;             // capacity of the position space
     uint32_t ntiles;           // tiles in use (end of the allocated tile range)
-    uint32_t ngroups;          // ceil(ntiles / 1024): groups of the two-level tile scan
+    uint32_t par;              // this substep's parity
     uint32_t chunk_cap;        // capacity of the chunk list
     uint32_t chunk;            // particles per chunk this substep (kChunk or kChunkSmall)
     const SceneDesc* scenes;
     const uint32_t* tile_scene;    // scene of each global tile (kHole: free)
     uint32_t* cell_count;      // total cells + 1, zero outside binning
-    uint32_t* cell_start;      // per cell: first position of its particles (local to the tile until finished)
+    uint32_t* cell_start;      // per cell: first position of its particles
     uint32_t* key;             // npos: binning cell (global) of each position of the current state, or kHole
     uint32_t* rank;            // npos: rank within the cell
     uint32_t* perm;            // npos: position -> position of the previous layout
     uint32_t* tile_flags;      // per tile
-    uint32_t* tile_occ;        // per tile: 1 if the tile holds particles this substep
-    uint32_t* tile_cnt;        // per tile: particles (occupied tiles)
-    uint32_t* tile_pstart;     // per tile: exclusive scan of tile_cnt inside its 1024-tile group
-    uint32_t* tile_cstart;     // per tile: exclusive scan of the chunk counts inside its group
-    uint32_t* group_pstart;    // per group: exclusive scan of the group particle totals
-    uint32_t* group_cstart;    // per group: exclusive scan of the group chunk totals
-    uint4* chunk_info;         // per chunk: (tile, first position, end position, first local cell)
-    uint32_t* chunk_last;      // per chunk: last local cell
-    uint4* chunk_hdr;          // per chunk, 2 words: the packed ChunkHdr (written by P2G_MASS)
-    uint4* chunk_geo;          // per chunk: (scene, tile x, tile y, tile z) of its tile
+    uint4* chunk_hdr;          // per chunk of this substep's layout, 2 words: the packed ChunkHdr (written by the binning)
+    const uint4* chunk_hdr_prev;   // the previous layout's
+    uint32_t* tile_cnt;        // per tile: particles for the next binning (counted by G2P and imports)
+    uint2* tile_base;          // per listed tile: its first position and chunk (worlds of many tiles)
     uint32_t* tile_occ_list;
     uint32_t* tile_grid_list;
     Ctrl* ctrl;
@@ -202,16 +194,9 @@ struct World {
     uint32_t* rank = nullptr;
     uint32_t* perm = nullptr;
     uint32_t* tile_flags = nullptr;
-    uint32_t* tile_occ = nullptr;
     uint32_t* tile_cnt = nullptr;
-    uint32_t* tile_pstart = nullptr;
-    uint32_t* tile_cstart = nullptr;
-    uint32_t* group_pstart = nullptr;
-    uint32_t* group_cstart = nullptr;
-    uint4* chunk_info = nullptr;
-    uint32_t* chunk_last = nullptr;
-    uint4* chunk_hdr = nullptr;
-    uint4* chunk_geo = nullptr;
+    uint2* tile_base = nullptr;
+    uint4* chunk_hdr[2] = {nullptr, nullptr};   // by parity
     uint32_t chunk_cap = 0;
     uint32_t chunk = kChunk;   // chunk size of the substep being enqueued
     uint32_t* tile_occ_list = nullptr;
