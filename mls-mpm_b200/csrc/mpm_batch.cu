@@ -387,8 +387,12 @@ mpm_status mpm_batch_download(mpm_batch* b, int32_t scene, mpm_buffer which, voi
             float* aff = (float*)(base + N * 32);
             float* mass = (float*)(base + N * 68);
             float* dens = (float*)(base + N * 72);
-            cudaError_t e = cudaMemsetAsync(dens, 0, N * 4, st);
-            if (e == cudaSuccess) e = world_export_scene(w, scene, pos, vel, aff, mass, dens);
+            // only the buffer asked for (a density that no substep has computed reads 0)
+            auto want = [&](mpm_buffer b, auto* p) { return which == b ? p : nullptr; };
+            cudaError_t e = which == MPM_BUF_DENSITY ? cudaMemsetAsync(dens, 0, N * 4, st) : cudaSuccess;
+            if (e == cudaSuccess)
+                e = world_export_scene(w, scene, want(MPM_BUF_POS, pos), want(MPM_BUF_VEL, vel), want(MPM_BUF_AFFINE, aff),
+                                       want(MPM_BUF_MASS, mass), want(MPM_BUF_DENSITY, dens));
             if (e != cudaSuccess) return bcuda(e, "export");
             if (which == MPM_BUF_POS) { src = pos; size = n * 16; }
             if (which == MPM_BUF_VEL) { src = vel; size = n * 16; }

@@ -183,23 +183,29 @@ static bool is_particle_buffer(mpm_buffer w) {
     return w == MPM_BUF_POS || w == MPM_BUF_VEL || w == MPM_BUF_AFFINE || w == MPM_BUF_MASS || w == MPM_BUF_DENSITY;
 }
 
-// Binned engine: bring the reference-layout particle buffers up to date.
-static cudaError_t sync_reference_buffers(Scene& s) {
-    if (s.engine != kEngineBinned || !s.ref_stale) return cudaSuccess;
-    cudaError_t e = world_export_scene(s.world, s.world_slot, s.pos, s.vel, s.aff, s.mass, s.dens);
-    if (e == cudaSuccess) s.ref_stale = false;
+static uint32_t buffer_bit(mpm_buffer w) { return 1u << (unsigned)w; }
+
+// Binned engine: bring the reference-layout particle buffers up to date, those
+// in `which` (the masses never change: they are the buffers the scene was
+// loaded from).
+static cudaError_t sync_reference_buffers(Scene& s, uint32_t which = kParticleState) {
+    const uint32_t need = s.ref_stale & which;
+    if (s.engine != kEngineBinned || !need) return cudaSuccess;
+    auto want = [&](mpm_buffer b) { return (need & buffer_bit(b)) != 0; };
+    cudaError_t e = world_export_scene(s.world, s.world_slot, want(MPM_BUF_POS) ? s.pos : nullptr,
+                                       want(MPM_BUF_VEL) ? s.vel : nullptr, want(MPM_BUF_AFFINE) ? s.aff : nullptr,
+                                       nullptr, want(MPM_BUF_DENSITY) ? s.dens : nullptr);
+    if (e == cudaSuccess) s.ref_stale &= ~need;
     return e;
 }
 
 // The buffers a renderer reads every frame (fluid-renderer.js:315-328).
 static bool render_buffer(mpm_buffer w) { return w == MPM_BUF_POS || w == MPM_BUF_VEL || w == MPM_BUF_DENSITY; }
 
-// Binned engine: make one reference-layout particle buffer current.  Once the
-// substeps mirror pos/vel/density (Scene::mirror), those three need nothing.
+// Binned engine: make one reference-layout particle buffer current.
 static cudaError_t ensure_reference(Scene& s, mpm_buffer which) {
-    if (s.engine != kEngineBinned || !is_particle_buffer(which)) return cudaSuccess;
-    if (s.mirror && render_buffer(which)) return cudaSuccess;
-    return sync_reference_buffers(s);
+    if (!is_particle_buffer(which)) return cudaSuccess;
+    return sync_reference_buffers(s, buffer_bit(which));
 }
 
 // Binned engine: (re)load the working state from the reference-layout buffers.
@@ -276,7 +282,8 @@ static cudaError_t launch_substep(Scene& s) {
     const cudaError_t ge = guard_top_history(s);
     if (ge != cudaSuccess) return ge;
     if (s.engine == kEnginePlain) return launch_substep_plain(s);
-    s.ref_stale = true;
+    // once the substeps mirror pos, vel and density, those three stay current
+    s.ref_stale |= s.mirror ? buffer_bit(MPM_BUF_AFFINE) : kParticleState;
     world_set_uniforms(s.world, s.world_slot, s.params, s.walls, &s.hand, s.hand_active, s.hand_dims);
     return world_substep(s.world, &s, true);
 }
@@ -471,7 +478,7 @@ mpm_status mpm_upload_particles(mpm_scene* sc, const float* pos4, const float* v
     s.n_active = n;
     s.params.particle_num = n;
     if (s.engine == kEngineBinned) {
-        s.ref_stale = false;
+        s.ref_stale = 0;
         CUDA_TRY(import_state(s), "import");
     }
     CUDA_TRY(cudaStreamSynchronize(st), "upload sync");
@@ -903,7 +910,7 @@ mpm_status mpm_raycast_fluid(mpm_scene* sc, const double origin[3], const double
     DeviceGuard guard(s.device);
     CUDA_TRY(ensure_edit_scratch(s, false), "raycast scratch");
     CUDA_TRY(flush_tail(s), "diffuse");
-    CUDA_TRY(sync_reference_buffers(s), "export");
+    CUDA_TRY(sync_reference_buffers(s, buffer_bit(MPM_BUF_POS)), "export");   // all the pass reads
     const mpm_ray_params ray = pack_ray(origin, dir, radius);
     CUDA_TRY(launch_raycast(ray, s.params.particle_num, s.pos, s.edit_word, s.stream), "raycast");
     s.launches += s.params.particle_num ? 1 : 0;

@@ -79,6 +79,9 @@ struct DiffuseState {
 // substep (MPM_FLAG_PLAIN), which mirrors the reference's dispatch list.
 enum Engine { kEngineBinned = 0, kEnginePlain = 1 };
 
+// The particle buffers a substep changes, as bits of Scene::ref_stale.
+constexpr uint32_t kParticleState = (1u << MPM_BUF_POS) | (1u << MPM_BUF_VEL) | (1u << MPM_BUF_AFFINE) | (1u << MPM_BUF_DENSITY);
+
 struct Scene {
     int device = 0;
     int engine = kEngineBinned;
@@ -112,7 +115,7 @@ struct Scene {
     World world;              // binned engine: a world holding this one scene
     int world_slot = -1;
     // binned engine: which copy of the particle state is newer
-    bool ref_stale = false;    // reference-layout buffers behind the binned state
+    uint32_t ref_stale = 0;    // bits (1 << mpm_buffer) of the reference-layout buffers behind the binned state
     bool fast_stale = false;   // binned state behind the reference-layout buffers
     // binned engine: pos, vel and density in the reference layout are written
     // by every substep (turned on by the first mpm_get_buffer of one of them,

@@ -194,25 +194,33 @@ __global__ void k_extend(WorldView v, uint32_t end) {
         v.key[p] = kHole;
 }
 
-// Writes a scene's particles to reference-layout buffers by local id.
+// Writes a scene's particles, which lie at positions [j0, j1), to
+// reference-layout buffers by local id; null outputs are left out.
 __global__ void k_export(WorldView v, const float4* __restrict__ posm, const float4* __restrict__ rows,
-                         const uint32_t* __restrict__ ids, const float* __restrict__ dens, uint32_t id0, uint32_t n,
-                         float4* __restrict__ pos, float4* __restrict__ vel, float* __restrict__ aff_out,
-                         float* __restrict__ mass, float* __restrict__ dens_out) {
-    const uint32_t total = min(v.ctrl->total_pos, v.npos);
+                         const uint32_t* __restrict__ ids, const float* __restrict__ dens, uint32_t j0, uint32_t j1,
+                         uint32_t id0, uint32_t n, float4* __restrict__ pos, float4* __restrict__ vel,
+                         float* __restrict__ aff_out, float* __restrict__ mass, float* __restrict__ dens_out) {
+    const uint32_t end = min(min(v.ctrl->total_pos, v.npos), j1);
     const size_t plane = v.npos;
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < total; j += gridDim.x * blockDim.x) {
+    for (uint32_t j = j0 + blockIdx.x * blockDim.x + threadIdx.x; j < end; j += gridDim.x * blockDim.x) {
         if (v.key[j] == kHole) continue;
         const uint32_t id = ids[j] - id0;
         if (id >= n) continue;
-        const float4 p = posm[j], r0 = rows[j], r1 = rows[plane + j], r2 = rows[2 * plane + j];
-        pos[id] = make_float4(p.x, p.y, p.z, 0.0f);
-        vel[id] = make_float4(r0.w, r1.w, r2.w, 0.0f);
-        mass[id] = p.w;
-        if (dens_out) dens_out[id] = dens[j];
-        const float a[9] = {r0.x, r0.y, r0.z, r1.x, r1.y, r1.z, r2.x, r2.y, r2.z};
+        if (pos || mass) {
+            const float4 p = posm[j];
+            if (pos) pos[id] = make_float4(p.x, p.y, p.z, 0.0f);
+            if (mass) mass[id] = p.w;
+        }
+        if (vel || aff_out) {
+            const float4 r0 = rows[j], r1 = rows[plane + j], r2 = rows[2 * plane + j];
+            if (vel) vel[id] = make_float4(r0.w, r1.w, r2.w, 0.0f);
+            if (aff_out) {
+                const float a[9] = {r0.x, r0.y, r0.z, r1.x, r1.y, r1.z, r2.x, r2.y, r2.z};
 #pragma unroll
-        for (int e = 0; e < 9; ++e) aff_out[9ull * id + e] = a[e];
+                for (int e = 0; e < 9; ++e) aff_out[9ull * id + e] = a[e];
+            }
+        }
+        if (dens_out) dens_out[id] = dens[j];
     }
 }
 
@@ -2279,6 +2287,7 @@ cudaError_t world_add_scene(World& w, uint32_t X, uint32_t Y, uint32_t Z, const 
         }
         e = cudaGetLastError();
         w.pos_bound = h_total + n;
+        w.dense = false;
     }
     w.n_total += n;
     *slot_out = slot;
@@ -2342,6 +2351,7 @@ cudaError_t world_remove_scene(World& w, int slot) {
     r = SceneRec();
     w.table_dirty = true;
     w.generation++;
+    w.dense = false;
     if (e == cudaSuccess) e = cudaGetLastError();
     return e;
 }
@@ -2350,9 +2360,17 @@ cudaError_t world_export_scene(World& w, int slot, float4* pos, float4* vel, flo
     const SceneRec& r = w.scenes[slot];
     if (!r.live || r.n == 0) return cudaSuccess;
     const WorldView v = w.view();
-    k_export<<<w.pos_blocks, 256, 0, w.stream>>>(v, w.posm[w.cur], w.rows[w.cur], w.pid[w.cur], w.dens,
-                                                      r.id_base, r.n, pos, vel, aff, mass,
-                                                      w.dens_valid ? dens : nullptr);
+    // After a substep the layout is dense and in the order of the tiles, so of
+    // the scenes' tile ranges; scenes added or removed since leave it open.
+    uint32_t j0 = 0, j1 = w.npos;
+    if (w.dense) {
+        for (const SceneRec& o : w.scenes)
+            if (o.live && o.tile_base < r.tile_base) j0 += o.n;
+        j1 = j0 + r.n;
+    }
+    k_export<<<std::min<uint32_t>(cdiv(j1 - j0, 256), w.pos_blocks), 256, 0, w.stream>>>(
+        v, w.posm[w.cur], w.rows[w.cur], w.pid[w.cur], w.dens, j0, j1, r.id_base, r.n, pos, vel, aff, mass,
+        w.dens_valid ? dens : nullptr);
     w.launches++;
     w.tbl_outside[w.cur] = true;
     return cudaGetLastError();
@@ -2469,6 +2487,7 @@ static cudaError_t enqueue_substep(World& w, Scene* ds, const RefOut& ro, bool t
     w.dens_valid = true;
     w.counted = true;   // G2P ranked every new position in its cell
     w.pos_bound = w.n_total;   // the layout after a substep is dense
+    w.dense = true;
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     if (dv.enabled) {
@@ -2594,6 +2613,7 @@ cudaError_t world_substep(World& w, Scene* ds, bool use_graph) {
         dsc->diffuse.tail_pending = true;   // this substep's tail waits for the next one
     }
     w.pos_bound = w.n_total;   // the layout after a substep is dense
+    w.dense = true;
     w.cm_current = w.grid_i32[w.gbuf];
     w.cur ^= 1;
     w.gbuf ^= 1;

@@ -160,6 +160,7 @@ struct World {
     // binning cell in rank/cell_count; adding or removing a scene clears it
     // and the next substep recounts (k_count)
     bool counted = false;
+    bool dense = false;   // the layout is the last substep's: no holes, scenes in the order of their tiles
     uint64_t launches = 0;
     uint64_t generation = 1;                // bumps whenever the captured launch arguments change
 
@@ -235,7 +236,8 @@ cudaError_t world_add_scene(World& w, uint32_t X, uint32_t Y, uint32_t Z, const 
                             const mpm_wall_params& W, const float4* pos, const float4* vel, const float* aff,
                             const float* mass, uint32_t n, int* slot);
 cudaError_t world_remove_scene(World& w, int slot);
-// Writes a scene's particles (reference layouts, by local id) to device buffers.
+// Writes a scene's particles (reference layouts, by local id) to device
+// buffers; null ones are left out.
 cudaError_t world_export_scene(World& w, int slot, float4* pos, float4* vel, float* aff, float* mass, float* dens);
 // Grid buffers of a scene (reference layouts) inside the world arrays.
 void world_scene_grid(const World& w, int slot, int32_t** cm, int32_t** mv, float** cmf, float** mvf);
