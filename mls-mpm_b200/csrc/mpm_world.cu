@@ -2543,8 +2543,21 @@ cudaError_t world_substep(World& w, Scene* ds, bool use_graph) {
     }
     const bool tail_in = diffuse && ds->diffuse.tail_pending;
     const bool defer = diffuse && !profiling;
+    // Capturing and instantiating a substep costs the host about 0.2 ms a graph
+    // (two parities), launching its kernels one by one about 20 us more than
+    // replaying: a graph pays off once its launch arguments last some
+    // kCaptureAfter substeps.  Worlds whose scenes change every few substeps
+    // (an editing user, a serving loop) are never captured.
+    constexpr uint32_t kCaptureAfter = 16;
+    if (w.generation_seen != w.generation) {
+        w.generation_seen = w.generation;
+        w.generation_age = 0;
+    }
+    const int p = 2 * w.cur + (tail_in ? 1 : 0);   // cur and gbuf flip together: graphs per parity
+    const bool captured = w.graph[p] && w.graph_gen[p] == w.generation;
     // a substep that must recount runs eagerly; the captured graphs never count
-    if (!use_graph || profiling || !w.counted) {
+    if (!use_graph || profiling || !w.counted || (!captured && w.generation_age < kCaptureAfter)) {
+        w.generation_age++;
         e = enqueue_substep(w, ds, ro, tail_in, defer);
         if (e == cudaSuccess) e = cudaEventRecord(w.sub_done[parity], w.stream);
         return e;
@@ -2552,7 +2565,6 @@ cudaError_t world_substep(World& w, Scene* ds, bool use_graph) {
     // the diffuse update joins the graph: its kernels read the uniforms from
     // device copies and the advect parameters from a device copy
     Scene* dsc = diffuse ? ds : nullptr;
-    const int p = 2 * w.cur + (tail_in ? 1 : 0);   // cur and gbuf flip together: graphs per parity
     const bool mirror = ro.enabled != 0;
     if (!w.graph[p] || w.graph_gen[p] != w.generation || w.graph_diffuse[p] != diffuse ||
         w.graph_mirror[p] != mirror) {

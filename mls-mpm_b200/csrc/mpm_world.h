@@ -163,6 +163,8 @@ struct World {
     bool dense = false;   // the layout is the last substep's: no holes, scenes in the order of their tiles
     uint64_t launches = 0;
     uint64_t generation = 1;                // bumps whenever the captured launch arguments change
+    uint64_t generation_seen = 0;           // generation of the last substep, and how many ran eagerly in it
+    uint32_t generation_age = 0;
 
     // device arrays
     // the device scene table, one copy per buffer parity: a substep of
