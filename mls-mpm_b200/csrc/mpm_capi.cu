@@ -109,7 +109,7 @@ static void free_scene(Scene& s) {
         s.mvf = nullptr;
         s.vel4 = nullptr;
     }
-    void* ptrs[] = {s.pos, s.vel, s.aff, s.mass, s.dens, s.grid_i32, s.cmf, s.mvf,
+    void* ptrs[] = {s.pos, s.vel, s.aff, s.mass, s.dens, s.mirror_where, s.grid_i32, s.cmf, s.mvf,
                     s.diffuse.pool, s.diffuse.free_list, s.diffuse.top, s.diffuse.spawn_bits,
                     s.diffuse.kill_bits, s.diffuse.alive_mask, s.diffuse.block_counts, s.diffuse.kill_counts,
                     s.diffuse.rank_state,
@@ -197,6 +197,18 @@ static cudaError_t sync_reference_buffers(Scene& s, uint32_t which = kParticleSt
                                        nullptr, want(MPM_BUF_DENSITY) ? s.dens : nullptr);
     if (e == cudaSuccess) s.ref_stale &= ~need;
     return e;
+}
+
+// Turns on the substeps' own writes of pos, vel and density in the reference
+// layout.  Large scenes get k_mirror's table here; without memory for it G2P
+// goes on writing the buffers, as it does in smaller scenes.
+static void start_mirror(Scene& s) {
+    s.mirror = true;
+    if (s.capacity < kMirrorGather) return;
+    if (dalloc(&s.mirror_where, (size_t)s.capacity * 4) != cudaSuccess) {
+        cudaGetLastError();
+        s.mirror_where = nullptr;
+    }
 }
 
 // The buffers a renderer reads every frame (fluid-renderer.js:315-328).
@@ -477,6 +489,7 @@ mpm_status mpm_upload_particles(mpm_scene* sc, const float* pos4, const float* v
     CUDA_TRY(cudaMemcpyAsync(s.mass, mass, (size_t)n * 4, cudaMemcpyHostToDevice, st), "upload mass");
     s.n_active = n;
     s.params.particle_num = n;
+    s.loaded_at = s.substeps_done;
     if (s.engine == kEngineBinned) {
         s.ref_stale = 0;
         CUDA_TRY(import_state(s), "import");
@@ -672,7 +685,7 @@ mpm_status mpm_get_buffer(mpm_scene* sc, mpm_buffer which, void** dev_ptr, size_
         // frame: from now on every substep writes those three in place
         if (s.engine == kEngineBinned && render_buffer(which) && !s.mirror) {
             CUDA_TRY(sync_reference_buffers(s), "export");
-            s.mirror = true;
+            start_mirror(s);
         }
     }
     return MPM_OK;
@@ -707,7 +720,7 @@ mpm_status mpm_get_ipc_handle(mpm_scene* sc, mpm_buffer which, void* handle, siz
         CUDA_TRY(ensure_reference(s, which), "export");
         if (s.engine == kEngineBinned && render_buffer(which) && !s.mirror) {   // as mpm_get_buffer
             CUDA_TRY(sync_reference_buffers(s), "export");
-            s.mirror = true;
+            start_mirror(s);
         }
     }
     CUdeviceptr base = 0;

@@ -79,6 +79,14 @@ struct DiffuseState {
 // substep (MPM_FLAG_PLAIN), which mirrors the reference's dispatch list.
 enum Engine { kEngineBinned = 0, kEnginePlain = 1 };
 
+// Render buffers by k_mirror (mpm_world.cu): scenes of at least this capacity,
+// more than this many substeps after their load.
+#ifndef MPM_MIRROR_GATHER
+#define MPM_MIRROR_GATHER 1500000
+#endif
+constexpr uint32_t kMirrorGather = MPM_MIRROR_GATHER;
+constexpr uint64_t kMirrorMixed = 64;
+
 // The particle buffers a substep changes, as bits of Scene::ref_stale.
 constexpr uint32_t kParticleState = (1u << MPM_BUF_POS) | (1u << MPM_BUF_VEL) | (1u << MPM_BUF_AFFINE) | (1u << MPM_BUF_DENSITY);
 
@@ -121,6 +129,8 @@ struct Scene {
     // by every substep (turned on by the first mpm_get_buffer of one of them,
     // the sign of a consumer that reads them every frame)
     bool mirror = false;
+    uint32_t* mirror_where = nullptr;   // large scenes: each id's position (k_mirror); null: G2P writes the buffers itself
+    uint64_t loaded_at = 0;             // substeps_done at the last mpm_upload_particles (ids in the order of the load)
     uint64_t substeps_done = 0;
     uint64_t launches = 0;
 

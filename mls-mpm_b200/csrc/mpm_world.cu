@@ -1718,6 +1718,27 @@ struct G2POut {
     uint32_t* group_counts;
 };
 
+// A mirror record, one 32-byte access (aligned: records are 2 words from the
+// start of a device allocation): x, y, z, density, then vx, vy, vz.  As two
+// 16-byte accesses the pass and G2P's stores took 584 -> 659 us at 8M.
+__device__ __forceinline__ void store_record(float4* r, f3 x, float density, f3 v) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(r), "f"(x.x), "f"(x.y), "f"(x.z),
+                 "f"(density), "f"(v.x), "f"(v.y), "f"(v.z), "f"(0.0f)
+                 : "memory");
+}
+__device__ __forceinline__ void load_record(const float4* r, float4& a, float4& b) {
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+                 : "l"(r)
+                 : "memory");
+}
+// Store with an L2 evict-last hint.
+__device__ __forceinline__ void keep_store(uint32_t* p, uint32_t x) {
+    uint64_t pol;
+    asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol));
+    asm volatile("st.global.L2::cache_hint.u32 [%0], %1, %2;" ::"l"(p), "r"(x), "l"(pol) : "memory");
+}
+
 // G2P epilogue of one particle (shaders.js:631-700): affine, advection and
 // boundary handling, the new state at position p, its binning key and tile
 // mark, and the diffuse spawn decision.  Returns the particle's rank within
@@ -1735,7 +1756,10 @@ __device__ __forceinline__ uint32_t g2p_store(const G2POut& o, const SceneDesc& 
     o.ids[p] = gid;
     if (mirror) {   // particle_pos/vel (shaders.js:703-704) and particle_density (shaders.js:314) by id
         const uint32_t id = gid - sd.id_base;
-        if (id < sd.n) {
+        if (ro.record) {   // k_mirror writes the buffers from these
+            store_record(ro.record + 2ull * p, np, density, nv);
+            if (id < sd.n) keep_store(ro.where + id, p);
+        } else if (id < sd.n) {
 #if MPM_MIRROR_KEEP
             // the scattered 16- and 4-byte writes by id fill 32-byte sectors
             // half or an eighth at a time: an evict-last hint keeps their L2
@@ -1967,6 +1991,38 @@ __global__ void __launch_bounds__(kChunkThreads, MPM_G2P_MINB) k_g2p_chunks(Worl
         sb ^= 1;
     }
     if (pend_p != kHole) v.rank[pend_p] = pend_rank;
+}
+
+// The render buffers of a large scene, by id: each particle's record is read
+// from its place in the layout, and the buffers are written in order.  Particles
+// mix with time, and G2P's own writes by id (two of 16 bytes and one of 4) then
+// hit DRAM as partial sectors, each read and written, where the buffers (36 bytes
+// a particle) outgrow L2.  One 32-byte record a particle is read a whole sector
+// at a time instead, found by a table (4 bytes a particle, written by id) that
+// stays in L2.  G2P with the buffers kept by its own writes / by this pass, us,
+// 5, 60 and 300 substeps after the load: 1M 65 78 67 / 77 87 73, 1.7M 99 120 135 /
+// 115 132 120, 2.5M 137 180 219 / 162 177 167, 8.4M 432 609 870 / 499 545 570.  So
+// it runs in scenes of kMirrorGather particles from kMirrorMixed substeps after
+// their load on.
+__global__ void __launch_bounds__(256) k_mirror(RefOut ro, uint32_t n) {
+    constexpr uint32_t kPer = 4;   // records in flight a thread
+    const uint32_t i0 = blockIdx.x * (256u * kPer) + threadIdx.x;
+    uint32_t at[kPer];
+    float4 a[kPer], b[kPer];
+#pragma unroll
+    for (uint32_t r = 0; r < kPer; ++r) at[r] = i0 + r * 256u < n ? ro.where[i0 + r * 256u] : 0u;
+#pragma unroll
+    for (uint32_t r = 0; r < kPer; ++r) {
+        load_record(ro.record + 2ull * at[r], a[r], b[r]);
+    }
+#pragma unroll
+    for (uint32_t r = 0; r < kPer; ++r) {
+        const uint32_t id = i0 + r * 256u;
+        if (id >= n) break;
+        __stcs(ro.pos + id, make_float4(a[r].x, a[r].y, a[r].z, 0.0f));
+        __stcs(ro.vel + id, make_float4(b[r].x, b[r].y, b[r].z, 0.0f));
+        __stcs(ro.dens + id, a[r].w);
+    }
 }
 
 inline uint32_t cdiv(uint64_t a, uint32_t b) { return (uint32_t)((a + b - 1) / b); }
@@ -2480,6 +2536,11 @@ static cudaError_t enqueue_substep(World& w, Scene* ds, const RefOut& ro, bool t
             k_g2p_chunks<kChunk><<<w.item_blocks, kChunkThreads, 0, st>>>(v, w.posm[cur], w.pid[cur], w.vel4, w.cmf,
                                                                         w.posm[nxt], w.rows[nxt], w.pid[nxt], dv, ro);
         w.launches++;
+        if (ro.record) {
+            const uint32_t n = w.scenes[ro.scene].n;
+            k_mirror<<<cdiv(n ? n : 1, 1024), 256, 0, st>>>(ro, n);
+            w.launches++;
+        }
     }
     w.cur = nxt;
     w.gbuf ^= 1;
@@ -2523,6 +2584,12 @@ cudaError_t world_substep(World& w, Scene* ds, bool use_graph) {
         ro.pos = ds->pos;
         ro.vel = ds->vel;
         ro.dens = ds->dens;
+        // the records go where the old rows were: P2G_MOM has read them, and the
+        // next substep's G2P writes that buffer anew
+        if (ds->mirror_where && ds->substeps_done - ds->loaded_at > kMirrorMixed) {
+            ro.record = w.rows[w.cur];
+            ro.where = ds->mirror_where;
+        }
     }
     // chunk size: one pass per chunk when full-size chunks would leave blocks
     // of the chunk kernels idle (a new size means new captured graphs)
@@ -2565,7 +2632,7 @@ cudaError_t world_substep(World& w, Scene* ds, bool use_graph) {
     // the diffuse update joins the graph: its kernels read the uniforms from
     // device copies and the advect parameters from a device copy
     Scene* dsc = diffuse ? ds : nullptr;
-    const bool mirror = ro.enabled != 0;
+    const int mirror = ro.record ? 2 : (ro.enabled ? 1 : 0);
     if (!w.graph[p] || w.graph_gen[p] != w.generation || w.graph_diffuse[p] != diffuse ||
         w.graph_mirror[p] != mirror) {
         if (w.graph[p]) {

@@ -116,6 +116,11 @@ struct RefOut {
     float4* pos;
     float4* vel;
     float* dens;
+    // large scenes: G2P leaves 2-word records by position (x, y, z, density;
+    // vx, vy, vz) and each id's position, and k_mirror writes the buffers
+    // (null: G2P writes them)
+    float4* record;
+    uint32_t* where;
 };
 
 // Host record of a scene in a world.
@@ -220,7 +225,7 @@ struct World {
     uint64_t graph_gen[kGraphs] = {};
     uint64_t graph_kernels[kGraphs] = {};    // kernels in each graph (launch accounting)
     bool graph_diffuse[kGraphs] = {};        // the graph includes the diffuse update of its scene
-    bool graph_mirror[kGraphs] = {};         // the graph writes the owner's reference-layout mirrors
+    int graph_mirror[kGraphs] = {};          // the graph keeps the owner's render buffers: 0 no, 1 in G2P, 2 by k_mirror
 
     WorldView view() const;
 };
