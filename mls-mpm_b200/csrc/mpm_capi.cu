@@ -901,7 +901,7 @@ mpm_status mpm_delete_near(mpm_scene* sc, const double origin[3], const double d
     CUDA_TRY(launch_compact(del, n, s.pos, s.vel, s.mass, s.edit_pos, s.edit_vel, s.edit_mass, s.edit_blocks,
                             s.edit_word, st),
              "compact");
-    s.launches += n ? 3 : 0;
+    s.launches += n ? compact_launches(n) : 0;
     CUDA_TRY(cudaMemcpyAsync(s.edit_host, s.edit_word, 4, cudaMemcpyDeviceToHost, st), "count readback");
     CUDA_TRY(cudaStreamSynchronize(st), "compact sync");
     const uint32_t m = *s.edit_host;

@@ -3,10 +3,14 @@
 // The reference compacts with one atomic counter (shaders.js:542), so its
 // survivor order depends on thread scheduling.  Here the survivors keep their
 // index order (a deterministic order the reference can also produce): one pass
-// counts survivors per block of kCompactTile particles, one block scans the
-// counts, and a third pass writes each survivor at its block offset plus its
-// rank inside the block (warp ballots).  All three passes stream the inputs
-// with coalesced 16-byte loads; the work is HBM-bound (68 B per particle).
+// counts survivors per block of kCompactTile particles, and a second writes
+// each survivor at its block offset plus its rank inside the block (warp
+// ballots).  A block adds up the counts before its own by itself up to
+// kSelfScanBlocks blocks; beyond, where those reads would grow with the square
+// of n, one block scans the counts in between.  Both passes stream the inputs
+// with coalesced 16-byte loads, a thread's eight particles in flight at once:
+// the work is HBM-bound (72 B per particle kept; the second read of the
+// positions comes from L2 as far as they fit).
 #include <cuda_runtime.h>
 
 #include "mpm_device.cuh"
@@ -28,18 +32,40 @@ __device__ __forceinline__ bool survives(const float4 q, const mpm_ray_params& d
     return !(ray_perp_dist(mk(q.x, q.y, q.z), mk(del.ox, del.oy, del.oz), mk(del.dx, del.dy, del.dz)) < del.radius);
 }
 
-__global__ void __launch_bounds__(kCompactThreads) k_compact_count(mpm_ray_params del, uint32_t n,
-                                                                   const float4* __restrict__ pos,
-                                                                   uint32_t* __restrict__ counts) {
-    const uint64_t base = (uint64_t)blockIdx.x * kCompactTile;
-    uint32_t total = 0;
+constexpr uint32_t kCompactWarps = kCompactThreads / 32;
+
+// The positions of this thread's kCompactRounds particles (index base + r *
+// kCompactThreads + thread) and which of them survive, as a ballot per round.
+__device__ __forceinline__ void compact_load(const mpm_ray_params& del, uint32_t n, uint64_t base,
+                                             const float4* __restrict__ pos, float4* q, uint32_t* keep) {
 #pragma unroll
     for (uint32_t r = 0; r < kCompactRounds; ++r) {
         const uint64_t p = base + r * kCompactThreads + threadIdx.x;
-        const bool keep = p < n && survives(pos[p], del);
-        total += (uint32_t)__syncthreads_count(keep);
+        q[r] = p < n ? pos[p] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
-    if (threadIdx.x == 0) counts[blockIdx.x] = total;
+#pragma unroll
+    for (uint32_t r = 0; r < kCompactRounds; ++r)
+        keep[r] = __ballot_sync(0xffffffffu,
+                                base + r * kCompactThreads + threadIdx.x < n && survives(q[r], del));
+}
+
+__global__ void __launch_bounds__(kCompactThreads) k_compact_count(mpm_ray_params del, uint32_t n,
+                                                                   const float4* __restrict__ pos,
+                                                                   uint32_t* __restrict__ counts) {
+    __shared__ uint32_t ws[kCompactWarps];
+    float4 q[kCompactRounds];
+    uint32_t keep[kCompactRounds];
+    compact_load(del, n, (uint64_t)blockIdx.x * kCompactTile, pos, q, keep);
+    uint32_t total = 0;
+#pragma unroll
+    for (uint32_t r = 0; r < kCompactRounds; ++r) total += __popc(keep[r]);
+    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = total;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        total = 0;
+        for (uint32_t w = 0; w < kCompactWarps; ++w) total += ws[w];
+        counts[blockIdx.x] = total;
+    }
 }
 
 // One block: exclusive scan of the per-block counts in place; the total goes
@@ -79,6 +105,8 @@ __global__ void __launch_bounds__(1024) k_compact_scan(uint32_t nblocks, uint32_
     if (threadIdx.x == 0) *count_dev = carry;
 }
 
+// counts: the survivors per block (scanned: their exclusive prefixes).
+template <bool kScanned>
 __global__ void __launch_bounds__(kCompactThreads) k_compact_write(mpm_ray_params del, uint32_t n,
                                                                    const float4* __restrict__ pos_in,
                                                                    const float4* __restrict__ vel_in,
@@ -86,38 +114,67 @@ __global__ void __launch_bounds__(kCompactThreads) k_compact_write(mpm_ray_param
                                                                    float4* __restrict__ pos_out,
                                                                    float4* __restrict__ vel_out,
                                                                    float* __restrict__ mass_out,
-                                                                   const uint32_t* __restrict__ offsets) {
-    __shared__ uint32_t wsum[kCompactThreads / 32];
+                                                                   const uint32_t* __restrict__ counts,
+                                                                   uint32_t* __restrict__ count_dev) {
+    __shared__ uint32_t wsum[kCompactRounds][kCompactWarps];
+    __shared__ uint32_t part[kCompactWarps];
     const uint64_t base = (uint64_t)blockIdx.x * kCompactTile;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    uint32_t off = offsets[blockIdx.x];
-#pragma unroll 1
-    for (uint32_t r = 0; r < kCompactRounds; ++r) {
-        const uint64_t p = base + r * kCompactThreads + threadIdx.x;
-        float4 q = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        bool keep = false;
-        if (p < n) {
-            q = pos_in[p];
-            keep = survives(q, del);
-        }
-        const uint32_t bal = __ballot_sync(0xffffffffu, keep);
-        if (lane == 0) wsum[wid] = __popc(bal);
-        __syncthreads();
-        uint32_t before = 0, round_total = 0;
+    const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+    float4 q[kCompactRounds];
+    uint32_t keep[kCompactRounds];
+    compact_load(del, n, base, pos_in, q, keep);
+    if (lane == 0) {
 #pragma unroll
-        for (int w = 0; w < (int)(kCompactThreads / 32); ++w) {
-            const uint32_t c = wsum[w];
-            if (w < wid) before += c;
-            round_total += c;
+        for (uint32_t r = 0; r < kCompactRounds; ++r) wsum[r][wid] = __popc(keep[r]);
+    }
+    uint32_t off = 0;
+    if (kScanned) {
+        off = counts[blockIdx.x];
+    } else {
+        for (uint32_t b = threadIdx.x; b < blockIdx.x; b += kCompactThreads) off += counts[b];
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) off += __shfl_xor_sync(0xffffffffu, off, d);
+        if (lane == 0) part[wid] = off;
+    }
+    __syncthreads();
+    if (!kScanned) {
+        off = 0;
+#pragma unroll
+        for (uint32_t w = 0; w < kCompactWarps; ++w) off += part[w];
+    }
+    // first places of this warp's rounds
+    uint32_t at[kCompactRounds];
+#pragma unroll
+    for (uint32_t r = 0; r < kCompactRounds; ++r) {
+#pragma unroll
+        for (uint32_t w = 0; w < kCompactWarps; ++w) {
+            if (w == wid) at[r] = off;
+            off += wsum[r][w];
         }
-        if (keep) {
-            const uint32_t idx = off + before + __popc(bal & ((1u << lane) - 1u));
-            pos_out[idx] = q;
-            vel_out[idx] = vel_in[p];
-            mass_out[idx] = mass_in[p];
+    }
+    if (!kScanned && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *count_dev = off;
+    // four rounds' velocities and masses in flight at a time
+#pragma unroll
+    for (uint32_t r0 = 0; r0 < kCompactRounds; r0 += 4) {
+        float4 v[4];
+        float m[4];
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) {
+            const uint64_t p = base + (r0 + k) * kCompactThreads + threadIdx.x;
+            if ((keep[r0 + k] >> lane) & 1u) {
+                v[k] = vel_in[p];
+                m[k] = mass_in[p];
+            }
         }
-        off += round_total;
-        __syncthreads();
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) {
+            if ((keep[r0 + k] >> lane) & 1u) {
+                const uint32_t idx = at[r0 + k] + __popc(keep[r0 + k] & ((1u << lane) - 1u));
+                pos_out[idx] = q[r0 + k];
+                vel_out[idx] = v[k];
+                mass_out[idx] = m[k];
+            }
+        }
     }
 }
 
@@ -146,9 +203,14 @@ cudaError_t launch_compact(const mpm_ray_params& del, uint32_t n, const float4* 
     if (n == 0) return cudaMemsetAsync(count_dev, 0, 4, stream);
     const uint32_t nblocks = (uint32_t)((n + (uint64_t)kCompactTile - 1) / kCompactTile);
     k_compact_count<<<nblocks, kCompactThreads, 0, stream>>>(del, n, pos_in, scratch);
-    k_compact_scan<<<1, 1024, 0, stream>>>(nblocks, scratch, count_dev);
-    k_compact_write<<<nblocks, kCompactThreads, 0, stream>>>(del, n, pos_in, vel_in, mass_in, pos_out, vel_out,
-                                                             mass_out, scratch);
+    if (nblocks <= kSelfScanBlocks) {
+        k_compact_write<false><<<nblocks, kCompactThreads, 0, stream>>>(del, n, pos_in, vel_in, mass_in, pos_out, vel_out,
+                                                                        mass_out, scratch, count_dev);
+    } else {
+        k_compact_scan<<<1, 1024, 0, stream>>>(nblocks, scratch, count_dev);
+        k_compact_write<true><<<nblocks, kCompactThreads, 0, stream>>>(del, n, pos_in, vel_in, mass_in, pos_out, vel_out,
+                                                                       mass_out, scratch, count_dev);
+    }
     return cudaGetLastError();
 }
 

@@ -15,6 +15,11 @@ constexpr uint32_t kCompactThreads = 256;
 constexpr uint32_t kCompactRounds = 8;
 constexpr uint32_t kCompactTile = kCompactThreads * kCompactRounds;
 
+// Blocks up to which a compaction block adds up the counts before its own
+// (2: count and write); beyond, a scan runs in between (3 launches).
+constexpr uint32_t kSelfScanBlocks = 4096;
+inline uint32_t compact_launches(uint64_t n) { return (n + kCompactTile - 1) / kCompactTile <= kSelfScanBlocks ? 2u : 3u; }
+
 // Scratch words the compaction needs for n particles: one survivor count per
 // block of kCompactTile particles.  Every word is written by the count pass
 // before any pass reads it, so the scratch needs no clearing between calls.
