@@ -424,8 +424,8 @@ mpm_status mpm_batch_get_info(mpm_batch* batch, mpm_batch_info* info);
 typedef struct mpm_server mpm_server;
 
 /* mpm_server_desc.flags: keep each job's final particle state (pos, vel,
- * density) on the host for mpm_server_download (costs a synchronous copy per
- * job; meant for checking results). */
+ * density) on the host for mpm_server_download (36 bytes a particle, copied
+ * when the job retires and held until the server is destroyed). */
 #define MPM_SERVER_KEEP_STATE 0x100u
 
 typedef struct mpm_server_desc {
@@ -460,8 +460,9 @@ mpm_status mpm_server_destroy(mpm_server* server);
 
 /* Queues a job.  params: grid dims and uniforms as mpm_set_params takes them
  * (particle_num replaced by n); host arrays are copied into page-locked host
- * memory (pageable if page-locking fails), held until the mpm_server_run
- * that admits the job returns, so admission uploads are asynchronous.
+ * memory (pageable if page-locking fails), so that admission uploads are
+ * asynchronous.  When the mpm_server_run that finishes the job returns, the
+ * server keeps up to 256 MB of that memory for later jobs.
  * MPM_ERR_CAPACITY if the job can never fit the server. */
 mpm_status mpm_server_submit(mpm_server* server, const mpm_params* params, const float* pos4, const float* vel4,
                              const float* mass, uint32_t n, uint32_t substeps, double arrival_s, int64_t* job);

@@ -105,6 +105,23 @@ cudaError_t batch_reserve_stage(mpm_batch* b, uint32_t n) {
     b->stage_bytes = bytes;
     return cudaSuccess;
 }
+
+// pos | vel | density of a scene through the staging buffer, where they lie
+// one behind the other as in dst: one export and one copy, stream-ordered (the
+// staging buffer's earlier and later users are on the same stream).
+cudaError_t batch_export_state(mpm_batch* b, int32_t scene, void* dst) {
+    World& w = b->w;
+    const size_t n = w.scenes[scene].n;
+    if (n == 0) return cudaSuccess;
+    cudaError_t e = batch_reserve_stage(b, (uint32_t)n);
+    if (e != cudaSuccess) return e;
+    float4* pos = reinterpret_cast<float4*>(b->stage);
+    float* dens = reinterpret_cast<float*>(pos + 2 * n);
+    e = cudaMemsetAsync(dens, 0, n * 4, w.stream);   // (a density that no substep has computed reads 0)
+    if (e == cudaSuccess) e = world_export_scene(w, scene, pos, pos + n, nullptr, nullptr, dens);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(dst, pos, n * 36, cudaMemcpyDeviceToHost, w.stream);
+    return e;
+}
 }  // namespace mpm
 
 namespace {

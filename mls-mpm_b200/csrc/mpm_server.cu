@@ -14,6 +14,7 @@
 
 #include <algorithm>
 #include <chrono>
+#include <cstdlib>
 #include <cstring>
 #include <deque>
 #include <memory>
@@ -31,27 +32,114 @@ void set_error(const std::string& msg);
 // particles without allocating then.
 cudaError_t batch_reserve_stage(mpm_batch* b, uint32_t n);
 uint32_t* batch_health_word(mpm_batch* b, int32_t scene);
+// Enqueues the copy of a scene's pos, vel and density (36 bytes a particle, in
+// this order) to the host block dst.
+cudaError_t batch_export_state(mpm_batch* b, int32_t scene, void* dst);
 }
 
 namespace {
 
 using Clock = std::chrono::steady_clock;
 
+// Host memory of a job: its inputs (pos, vel if given, mass) until they are
+// uploaded at admission, then its final state (pos, vel, density) if it is kept.
+// Page-locked, so that both copies are asynchronous and the serving loop never
+// blocks on them while the device runs out of queued substeps; plain memory if
+// page-locking fails, and the copies then block.
+struct Block {
+    float* p = nullptr;
+    size_t bytes = 0;
+    bool pinned = false;
+};
+
+// The free blocks of one server.  Page-locking is what a submission spends its
+// time on: ten jobs of 0.3 to 3.6 MB (11 MB) take 16 ms to submit into new
+// blocks, 1.1 ms into blocks at hand.  So a run's blocks serve the next run's
+// jobs, up to kKeep bytes of them.
+class BlockPool {
+    static constexpr size_t kKeep = (size_t)256 << 20;
+    std::vector<Block> free_;
+    size_t bytes_ = 0;
+
+    static void destroy(Block& b) {
+        if (b.pinned) {
+            if (cudaFreeHost(b.p) != cudaSuccess) cudaGetLastError();
+        } else {
+            std::free(b.p);
+        }
+        b = Block{};
+    }
+
+public:
+    // The smallest free block that holds `need` bytes, if it is at most twice
+    // as large; otherwise a new one (sizes of four steps to the power of two,
+    // from 64 KB).  p == nullptr: out of memory.
+    Block take(size_t need) {
+        size_t pick = free_.size();
+        for (size_t i = 0; i < free_.size(); ++i)
+            if (free_[i].bytes >= need && free_[i].bytes / 2 <= std::max(need, (size_t)32 << 10) &&
+                (pick == free_.size() || free_[i].bytes < free_[pick].bytes))
+                pick = i;
+        Block b;
+        if (pick < free_.size()) {
+            b = free_[pick];
+            free_[pick] = free_.back();
+            free_.pop_back();
+            bytes_ -= b.bytes;
+            return b;
+        }
+        size_t unit = (size_t)16 << 10;
+        while (unit * 8 < need) unit *= 2;
+        b.bytes = std::max((need + unit - 1) / unit, (size_t)4) * unit;
+        void* p = nullptr;
+        b.pinned = cudaMallocHost(&p, b.bytes) == cudaSuccess;
+        if (!b.pinned) {
+            cudaGetLastError();   // clear the error: the pageable path still works
+            p = std::malloc(b.bytes);
+        }
+        b.p = static_cast<float*>(p);
+        return b;
+    }
+    // Back to the pool (only once no copy from or to it can be in flight).
+    void give(Block& b) {
+        if (!b.p) return;
+        if (!b.pinned || bytes_ + b.bytes > kKeep) return destroy(b);
+        try {
+            free_.push_back(b);
+        } catch (const std::bad_alloc&) {
+            return destroy(b);
+        }
+        bytes_ += b.bytes;
+        b = Block{};
+    }
+    void clear() {
+        for (Block& b : free_) destroy(b);
+        free_.clear();
+        bytes_ = 0;
+    }
+};
+
 struct Job {
     mpm_params P{};
-    std::vector<float> pos, vel, mass;   // page-locked while the job waits (pinned = true)
-    bool pinned = false;
+    Block block;                     // pos | vel | mass of n particles, from retirement on pos | vel | density
+    bool has_vel = false;
     uint32_t n = 0, substeps = 0, left = 0;
     double arrival = 0.0, admit = -1.0;
     volatile double finish = -1.0;   // written by the stream-ordered host function
     int32_t sid = -1;
     int state = 0;                   // 0 queued, 1 active, 2 done
-    std::vector<float> out_pos, out_vel, out_dens;
+    std::unique_ptr<float[]> out;    // pos | vel | density (MPM_SERVER_KEEP_STATE)
+    size_t out_done = 0;             // bytes of it moved from the block so far
+    uint64_t retired = 0;            // substeps enqueued when the job was retired
     const Clock::time_point* t0 = nullptr;
     // the scene's health bits, copied at retirement into a pinned slot and
     // from there into `health` by the stream-ordered host function
     const volatile uint32_t* health_slot = nullptr;
     volatile uint32_t health = 0;
+
+    size_t state_bytes() const { return (size_t)n * 36; }
+    float* vel_in() const { return block.p + (size_t)n * 4; }
+    float* mass_in() const { return block.p + (size_t)n * (has_vel ? 8 : 4); }
 };
 
 void CUDART_CB stamp_finish(void* p) {
@@ -65,39 +153,20 @@ mpm_status sfail(mpm_status st, const std::string& msg) {
     return st;
 }
 
-// A job's input arrays are page-locked when it is submitted, so its upload at
-// admission is an asynchronous copy: the serving loop never blocks on it
-// while the device runs out of queued substeps.  Without page-locking the
-// upload still works, as a copy from pageable memory.
-void pin_inputs(Job& j) {
-    bool ok = true;
-    for (std::vector<float>* v : {&j.pos, &j.vel, &j.mass}) {
-        if (v->empty()) continue;
-        if (cudaHostRegister(v->data(), v->size() * sizeof(float), cudaHostRegisterDefault) != cudaSuccess) {
-            cudaGetLastError();   // clear the error: the pageable path still works
-            ok = false;
-        }
-    }
-    if (ok) {
-        j.pinned = true;
-        return;
-    }
-    for (std::vector<float>* v : {&j.pos, &j.vel, &j.mass})
-        if (!v->empty() && cudaHostUnregister(v->data()) != cudaSuccess) cudaGetLastError();
+// Moves up to `limit` bytes of a retired job's state from its block to `out`;
+// true when all of it is there.
+bool collect(Job& j, size_t limit) {
+    const size_t m = std::min(limit, j.state_bytes() - j.out_done);
+    std::memcpy(reinterpret_cast<char*>(j.out.get()) + j.out_done, reinterpret_cast<char*>(j.block.p) + j.out_done, m);
+    j.out_done += m;
+    return j.out_done == j.state_bytes();
 }
 
-// Release the inputs of an admitted job (only once no copy from them can be
-// in flight: after a stream synchronisation).
-void release_inputs(Job& j) {
-    if (j.pinned) {
-        for (std::vector<float>* v : {&j.pos, &j.vel, &j.mass})
-            if (!v->empty()) cudaHostUnregister(v->data());
-        j.pinned = false;
-    }
-    std::vector<float>().swap(j.pos);
-    std::vector<float>().swap(j.vel);
-    std::vector<float>().swap(j.mass);
-}
+// A retired job's state leaves its block a piece after each enqueued substep,
+// while the device works: a piece takes about 0.1 ms, most of it for the first
+// touch of the new pages, and a substep of the scenes that are served as long.
+// (The ten jobs' run: 20 ms with a waiting copy at each retirement, 8.1 ms so.)
+constexpr size_t kCollectPiece = (size_t)256 << 10;
 
 double percentile(std::vector<double> v, double q) {
     if (v.empty()) return 0.0;
@@ -118,6 +187,7 @@ struct mpm_server {
     uint64_t pcap = 0, ccap = 0;
     uint32_t scap = 0;
     std::vector<std::unique_ptr<Job>> jobs;
+    BlockPool pool;
     Clock::time_point t0;
     // pinned ring of health words copied at job retirement; a slot is reused
     // only after ring_size later retirements, by which time the host function
@@ -186,7 +256,8 @@ mpm_status mpm_server_create(const mpm_server_desc* d, mpm_server** out) {
 mpm_status mpm_server_destroy(mpm_server* s) {
     if (!s) return MPM_OK;
     mpm_batch_destroy(s->batch);   // waits for the batch's stream
-    for (auto& j : s->jobs) release_inputs(*j);
+    for (auto& j : s->jobs) s->pool.give(j->block);
+    s->pool.clear();
     if (s->health_ring) cudaFreeHost(s->health_ring);
     delete s;
     return MPM_OK;
@@ -206,15 +277,20 @@ mpm_status mpm_server_submit(mpm_server* s, const mpm_params* P, const float* po
     j->n = n;
     j->substeps = j->left = substeps;
     j->arrival = arrival_s;
-    j->pos.assign(pos4, pos4 + (size_t)n * 4);
-    if (vel4) j->vel.assign(vel4, vel4 + (size_t)n * 4);
-    j->mass.assign(mass, mass + n);
     {
         int prev = -1;
         cudaGetDevice(&prev);
         cudaSetDevice(s->device);
-        pin_inputs(*j);
+        const bool full = vel4 || (s->flags & MPM_SERVER_KEEP_STATE);
+        j->block = s->pool.take((size_t)n * (full ? 36 : 20));
         if (prev >= 0) cudaSetDevice(prev);
+    }
+    if (!j->block.p) return sfail(MPM_ERR_OOM, "host allocation");
+    j->has_vel = vel4 != nullptr;
+    if (n) {
+        std::memcpy(j->block.p, pos4, (size_t)n * 16);
+        if (vel4) std::memcpy(j->vel_in(), vel4, (size_t)n * 16);
+        std::memcpy(j->mass_in(), mass, (size_t)n * 4);
     }
     j->t0 = &s->t0;
     *job = (int64_t)s->jobs.size();
@@ -262,6 +338,7 @@ mpm_status mpm_server_run(mpm_server* s, mpm_server_stats* stats) {
         if (mpm::batch_reserve_stage(s->batch, nmax) != cudaSuccess) return sfail(MPM_ERR_OOM, "staging allocation");
     }
     std::vector<Job*> active;
+    std::deque<Job*> retired;   // their states are on the way to their blocks, or there and not yet moved on
     uint64_t k = 0, updates = 0, active_sum = 0, active_max = 0;
     const bool keep = (s->flags & MPM_SERVER_KEEP_STATE) != 0;
     s->t0 = Clock::now();
@@ -272,14 +349,13 @@ mpm_status mpm_server_run(mpm_server* s, mpm_server_stats* stats) {
         while (!queue.empty() && queue.front()->arrival <= t) {
             Job* j = queue.front();
             int32_t sid = -1;
-            const mpm_status st = mpm_batch_add(s->batch, &j->P, nullptr, j->pos.data(),
-                                                j->vel.empty() ? nullptr : j->vel.data(), nullptr, j->mass.data(),
-                                                j->n, &sid);
+            const mpm_status st = mpm_batch_add(s->batch, &j->P, nullptr, j->block.p,
+                                                j->has_vel ? j->vel_in() : nullptr, nullptr, j->mass_in(), j->n, &sid);
             if ((st == MPM_ERR_BUSY || st == MPM_ERR_CAPACITY) && !active.empty()) break;   // wait for retirements
             if (st != MPM_OK) return st;   // an empty batch that cannot take the job never will
             j->sid = sid;
             j->admit = t;
-            j->state = 1;   // its inputs are released after the final synchronisation
+            j->state = 1;   // its block goes back to the pool after the final synchronisation
             queue.pop_front();
             active.push_back(j);
         }
@@ -313,26 +389,34 @@ mpm_status mpm_server_run(mpm_server* s, mpm_server_stats* stats) {
             j->health_slot = slot_h;
             if (cudaLaunchHostFunc(stream, stamp_finish, j) != cudaSuccess) return sfail(MPM_ERR_DEVICE, "host func");
             if (keep) {
-                j->out_pos.resize((size_t)j->n * 4);
-                j->out_vel.resize((size_t)j->n * 4);
-                j->out_dens.resize(j->n);
-                st = mpm_batch_download(s->batch, j->sid, MPM_BUF_POS, j->out_pos.data(), (size_t)j->n * 16);
-                if (st == MPM_OK)
-                    st = mpm_batch_download(s->batch, j->sid, MPM_BUF_VEL, j->out_vel.data(), (size_t)j->n * 16);
-                if (st == MPM_OK)
-                    st = mpm_batch_download(s->batch, j->sid, MPM_BUF_DENSITY, j->out_dens.data(), (size_t)j->n * 4);
-                if (st != MPM_OK) return st;
+                j->out.reset(new (std::nothrow) float[(size_t)j->n * 9 + 1]);
+                if (!j->out) return sfail(MPM_ERR_OOM, "host allocation");
+                if (mpm::batch_export_state(s->batch, j->sid, j->block.p) != cudaSuccess)
+                    return sfail(MPM_ERR_DEVICE, "state copy");
+                j->retired = k;
+                retired.push_back(j);
             }
             st = mpm_batch_remove(s->batch, j->sid);
             if (st != MPM_OK) return st;
-            j->state = 2;
+            if (!keep) j->state = 2;
             updates += (uint64_t)j->n * j->substeps;
         }
         active.resize(w);
+        // The event of substep q, waited for above at k = q + R (k counts this
+        // substep by now), has the copies of all jobs before it that retired
+        // with q substeps or fewer enqueued.
+        if (!retired.empty() && retired.front()->retired + R < k && collect(*retired.front(), kCollectPiece)) {
+            retired.front()->state = 2;
+            retired.pop_front();
+        }
     }
     if (cudaStreamSynchronize(stream) != cudaSuccess) return sfail(MPM_ERR_DEVICE, "final sync");
+    for (Job* j : retired) {
+        collect(*j, j->state_bytes());
+        j->state = 2;
+    }
     for (Job* j : this_run)
-        if (j->state != 0) release_inputs(*j);
+        if (j->state == 2) s->pool.give(j->block);
     if (stats) {
         std::memset(stats, 0, sizeof *stats);
         std::vector<double> lat;
@@ -385,13 +469,15 @@ mpm_status mpm_server_download(mpm_server* s, int64_t job, mpm_buffer which, voi
     const Job& j = *s->jobs[(size_t)job];
     if (j.state != 2 || !(s->flags & MPM_SERVER_KEEP_STATE))
         return sfail(MPM_ERR_INVALID_ARG, "job not finished or state not kept");
-    const std::vector<float>* v = which == MPM_BUF_POS ? &j.out_pos
-                                  : which == MPM_BUF_VEL ? &j.out_vel
-                                  : which == MPM_BUF_DENSITY ? &j.out_dens
-                                                             : nullptr;
-    if (!v) return sfail(MPM_ERR_INVALID_ARG, "only pos, vel and density are kept");
-    if (bytes > v->size() * 4) return sfail(MPM_ERR_INVALID_ARG, "bytes exceeds buffer size");
-    std::memcpy(host, v->data(), bytes);
+    size_t off, size;   // in floats, see Job::out
+    switch (which) {
+        case MPM_BUF_POS: off = 0; size = (size_t)j.n * 4; break;
+        case MPM_BUF_VEL: off = (size_t)j.n * 4; size = (size_t)j.n * 4; break;
+        case MPM_BUF_DENSITY: off = (size_t)j.n * 8; size = j.n; break;
+        default: return sfail(MPM_ERR_INVALID_ARG, "only pos, vel and density are kept");
+    }
+    if (bytes > size * 4) return sfail(MPM_ERR_INVALID_ARG, "bytes exceeds buffer size");
+    if (bytes) std::memcpy(host, j.out.get() + off, bytes);
     return MPM_OK;
 }
 
