@@ -15,6 +15,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstddef>
 #include <cstdint>
 
 #include "mpm_device.cuh"
@@ -443,6 +444,12 @@ __global__ void __launch_bounds__(kThreads) k_diffuse_gen_eval(const float4* __r
 // Diffuse ADVECT (shaders.js:858-997).  Kills set alive = 0 and a bit per
 // slot; k_freelist_pass (mode 1) then pushes killed slots in ascending slot
 // order (the order a one-at-a-time kill_particle, shaders.js:914-918, produces).
+// Bound by the 27 grid reads of a foam particle: slots lie in no spatial order,
+// so a warp's reads of one stencil cell hit some 10 lines.  Records move as three
+// 16-byte words (12 scalar accesses at a stride of 48 bytes cost as much as the
+// stencil) and a plane's reads are in flight together; with the kill pass 74 -> 64
+// us for 1M slots, 32 -> 28 us for 262,144.  Two 32-byte loads a row instead of
+// three of 16 were slower (71 us), as were 80 or 48 registers (67, 66).
 // ---------------------------------------------------------------------------
 // vel4 (binned engine): the same velocities as float4, one 16-byte load per cell.
 __device__ __forceinline__ f3 sample_grid_velocity(const float* __restrict__ mvf, const float4* __restrict__ vel4,
@@ -458,6 +465,29 @@ __device__ __forceinline__ f3 sample_grid_velocity(const float* __restrict__ mvf
     qweights(fy, wy[0], wy[1], wy[2]);
     qweights(fz, wz[0], wz[1], wz[2]);
     f3 v = mk(0.0f, 0.0f, 0.0f);
+    if (vel4 && cx >= 1 && cy >= 1 && cz >= 1 && cx + 1 < X && cy + 1 < Y && cz + 1 < Z) {
+        // the whole stencil lies in the grid: a plane's nine loads are issued
+        // before the first is used, at offsets from one cell
+        const float4* c0 = vel4 + ((uint32_t)(cz - 1) * (uint32_t)Y + (uint32_t)(cy - 1)) * (uint32_t)X + (uint32_t)(cx - 1);
+#pragma unroll
+        for (int k = 0; k < 3; ++k, c0 += (size_t)X * (uint32_t)Y) {
+            float4 c[9];
+#pragma unroll
+            for (int j = 0; j < 3; ++j)
+#pragma unroll
+                for (int i = 0; i < 3; ++i) c[3 * j + i] = c0[(uint32_t)(j * X + i)];
+#pragma unroll
+            for (int j = 0; j < 3; ++j)
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    const float w = wx[i] * wy[j] * wz[k];
+                    v.x += w * c[3 * j + i].x;
+                    v.y += w * c[3 * j + i].y;
+                    v.z += w * c[3 * j + i].z;
+                }
+        }
+        return v;
+    }
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         const int32_t zz = cz - 1 + k;
@@ -494,6 +524,27 @@ __device__ __forceinline__ void reflect_axis(float& p, float& v, float lo, float
     v = nv;
 }
 
+// A slot's record as three 16-byte words (device allocations and 48-byte
+// strides keep every record 16-byte aligned).
+static_assert(sizeof(mpm_diffuse_particle) == 48 && offsetof(mpm_diffuse_particle, vel) == 16 &&
+                  offsetof(mpm_diffuse_particle, ptype) == 32 && offsetof(mpm_diffuse_particle, lifetime) == 40,
+              "record layout");
+__device__ __forceinline__ mpm_diffuse_particle load_record(const mpm_diffuse_particle* __restrict__ src) {
+    const float4* q = reinterpret_cast<const float4*>(src);
+    const float4 a = q[0], b = q[1], c = q[2];
+    mpm_diffuse_particle p;
+    p.pos[0] = a.x; p.pos[1] = a.y; p.pos[2] = a.z; p.pos[3] = a.w;
+    p.vel[0] = b.x; p.vel[1] = b.y; p.vel[2] = b.z; p.vel[3] = b.w;
+    p.ptype = __float_as_uint(c.x); p.alive = __float_as_uint(c.y); p.lifetime = c.z; p._pad = c.w;
+    return p;
+}
+__device__ __forceinline__ void store_record(mpm_diffuse_particle* __restrict__ dst, const mpm_diffuse_particle& p) {
+    float4* q = reinterpret_cast<float4*>(dst);
+    q[0] = make_float4(p.pos[0], p.pos[1], p.pos[2], p.pos[3]);
+    q[1] = make_float4(p.vel[0], p.vel[1], p.vel[2], p.vel[3]);
+    q[2] = make_float4(__uint_as_float(p.ptype), __uint_as_float(p.alive), p.lifetime, p._pad);
+}
+
 __device__ __forceinline__ void diffuse_advect(mpm_diffuse_particle* __restrict__ pool, const float* __restrict__ mvf,
                                                const float4* __restrict__ vel4, const mpm_params& P,
                                                const mpm_advect_params& adv, const mpm_wall_params& W,
@@ -507,7 +558,7 @@ __device__ __forceinline__ void diffuse_advect(mpm_diffuse_particle* __restrict_
     const uint32_t word = (i >> 5) < nwords ? alive_mask[i >> 5] : 0u;
     bool kill = false;
     if (i < M && ((word >> (i & 31u)) & 1u)) {
-        mpm_diffuse_particle p = pool[i];
+        mpm_diffuse_particle p = load_record(pool + i);
         const f3 pos3 = mk(p.pos[0], p.pos[1], p.pos[2]);
         const float dt = P.dt, g = P.gravity;
         bool dead = false;
@@ -515,18 +566,18 @@ __device__ __forceinline__ void diffuse_advect(mpm_diffuse_particle* __restrict_
             p.vel[1] += g * dt;
             p.pos[0] = pos3.x + dt * p.vel[0]; p.pos[1] = pos3.y + dt * p.vel[1]; p.pos[2] = pos3.z + dt * p.vel[2];
             p.pos[3] = 0.0f;
-        } else if (p.ptype == MPM_DIFFUSE_FOAM) {
+        } else if (p.ptype == MPM_DIFFUSE_FOAM || p.ptype == MPM_DIFFUSE_BUBBLE) {
             const f3 gv = sample_grid_velocity(mvf, vel4, P, pos3);
-            p.pos[0] = pos3.x + dt * gv.x; p.pos[1] = pos3.y + dt * gv.y; p.pos[2] = pos3.z + dt * gv.z;
-            p.pos[3] = 0.0f;
-            p.lifetime -= dt;
-            if (p.lifetime <= 0.0f) dead = true;
-        } else if (p.ptype == MPM_DIFFUSE_BUBBLE) {
-            const f3 gv = sample_grid_velocity(mvf, vel4, P, pos3);
-            p.vel[0] += dt * adv.drag * (gv.x - p.vel[0]);
-            p.vel[1] += dt * (adv.buoyancy * -g + adv.drag * (gv.y - p.vel[1]));
-            p.vel[2] += dt * adv.drag * (gv.z - p.vel[2]);
-            p.pos[0] = pos3.x + dt * p.vel[0]; p.pos[1] = pos3.y + dt * p.vel[1]; p.pos[2] = pos3.z + dt * p.vel[2];
+            if (p.ptype == MPM_DIFFUSE_FOAM) {
+                p.pos[0] = pos3.x + dt * gv.x; p.pos[1] = pos3.y + dt * gv.y; p.pos[2] = pos3.z + dt * gv.z;
+                p.lifetime -= dt;
+                if (p.lifetime <= 0.0f) dead = true;
+            } else {
+                p.vel[0] += dt * adv.drag * (gv.x - p.vel[0]);
+                p.vel[1] += dt * (adv.buoyancy * -g + adv.drag * (gv.y - p.vel[1]));
+                p.vel[2] += dt * adv.drag * (gv.z - p.vel[2]);
+                p.pos[0] = pos3.x + dt * p.vel[0]; p.pos[1] = pos3.y + dt * p.vel[1]; p.pos[2] = pos3.z + dt * p.vel[2];
+            }
             p.pos[3] = 0.0f;
         }
         if (!dead) {
@@ -561,7 +612,7 @@ __device__ __forceinline__ void diffuse_advect(mpm_diffuse_particle* __restrict_
             reflect_axis(p.pos[2], p.vel[2], P.hard_min, P.hard_max_z);
             p.pos[3] = 0.0f;
             p.vel[3] = 0.0f;
-            pool[i] = p;
+            store_record(pool + i, p);
         }
     }
     const unsigned b = __ballot_sync(0xffffffffu, kill);
@@ -618,20 +669,29 @@ __global__ void __launch_bounds__(kThreads) k_alive_mask_build(const mpm_diffuse
 // (shaders.js:789-798 try_spawn, shaders.js:914-918 kill_particle), taken one
 // at a time in ascending id order.  Mode 0 (spawn): the spawner of rank r
 // takes free_list[top-1-r] while r < min(total, top).  Mode 1 (kill): the
-// killed slot of rank r goes to free_list[top+r].  Block b owns the
-// contiguous groups [b*R, (b+1)*R); every block reads all counts (a few KB)
-// for its prefix and the total, so no block waits on another.  One warp per
-// group: the group's 8 bitmap words are taken in ascending order, lane l
-// holding bit l of the word.  state = {top before, total, applied, ticket}:
+// killed slot of rank r goes to free_list[top+r].  Every block reads all
+// counts (4 bytes per 256 ids) and keeps the counts before each segment of
+// 64 << seg_shift groups, so no block waits on another and a warp finds the
+// count before any group from its segment's.  One warp per group, neighbouring
+// groups on neighbouring warps of all blocks: when the pool fills up, only the
+// spawners of low ids find a slot, and in contiguous shares (each block its
+// own run of groups) a quarter of the blocks then had all the work.  A group's
+// 8 bitmap words are taken in ascending order, lane l holding bit l of the
+// word.  What bounds it is latency (the chain counts, bits, free list, record)
+// while few ids spawn or die, and the scattered 48-byte records when many do:
+// per substep of 230k, 1M and 8M particles with 30,000, 262,144 and 1M slots the
+// spawn passes take 11, 17 and 36 us on average, in contiguous shares with two
+// records a lane in flight 14, 16 and 55.
+// state = {top before, total, applied, ticket}:
 // the last block to finish (ticket) writes the new top and resets the ticket;
 // a kill pass also appends the new top to top_hist (state[4] counts them) and
 // clears the spawn bits and counts (clear_bits, clear_counts) that the spawn
 // pass before it read, ready for the next substep's G2P.
 constexpr int kPassThreads = 512;
-constexpr uint32_t kNoSlot = 0xFFFFFFFFu;
+constexpr uint32_t kSegGroups = 64, kMaxSegs = 512;
 __global__ void __launch_bounds__(kPassThreads, 2) k_freelist_pass(const uint32_t* __restrict__ bits, uint32_t nbits,
                                                                 const uint32_t* __restrict__ counts, uint32_t ng,
-                                                                uint32_t R, int32_t* __restrict__ top,
+                                                                uint32_t seg_shift, int32_t* __restrict__ top,
                                                                 int32_t* __restrict__ state,
                                                                 uint32_t* __restrict__ free_list,
                                                                 const mpm_diffuse_particle* __restrict__ staging,
@@ -642,130 +702,121 @@ __global__ void __launch_bounds__(kPassThreads, 2) k_freelist_pass(const uint32_
                                                                 uint32_t nclear_counts,
                                                                 uint32_t* __restrict__ alive_mask) {
     constexpr int kWarps = kPassThreads / 32;
-    __shared__ uint32_t red[2][kWarps];
-    __shared__ uint32_t excl[kPassThreads];
+    static_assert(kMaxSegs == kPassThreads, "the scan takes one segment a thread");
+    __shared__ uint32_t red[kWarps];
+    __shared__ uint32_t seg[kMaxSegs];     // a segment's count, then the count before it
+    __shared__ uint8_t member[kWarps][kGroupIds];        // (spawn) a group's spawners in rank order
     __shared__ int32_t s_t0;
     const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
-    const uint32_t g0 = blockIdx.x * R, g1 = min(ng, g0 + R);
-    if (threadIdx.x == 0) s_t0 = *top;
-    // the total and the count before this block's first group
-    uint32_t all = 0, before = 0;
-    {
-        const uint32_t n4 = ng / 4;   // counts is 16-byte aligned (a device allocation)
-        const uint4* c4 = reinterpret_cast<const uint4*>(counts);
-        for (uint32_t i = threadIdx.x; i < n4; i += kPassThreads) {
-            const uint4 c = c4[i];
-            const uint32_t g = 4 * i;
-            all += c.x + c.y + c.z + c.w;
-            before += (g < g0 ? c.x : 0u) + (g + 1 < g0 ? c.y : 0u) + (g + 2 < g0 ? c.z : 0u) + (g + 3 < g0 ? c.w : 0u);
-        }
-        for (uint32_t g = 4 * n4 + threadIdx.x; g < ng; g += kPassThreads) {
-            const uint32_t c = counts[g];
-            all += c;
-            if (g < g0) before += c;
-        }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        all += __shfl_xor_sync(0xffffffffu, all, o);
-        before += __shfl_xor_sync(0xffffffffu, before, o);
-    }
-    if (lane == 0) { red[0][wid] = all; red[1][wid] = before; }
-    __syncthreads();
-    all = 0;
-    before = 0;
-    for (int k = 0; k < kWarps; ++k) { all += red[0][k]; before += red[1][k]; }
-    const int32_t t0 = s_t0, total = (int32_t)all;
-    const int32_t applied = mode == 0 ? (t0 > 0 ? (total < t0 ? total : t0) : 0) : total;
     const uint32_t nwords = (nbits + 31u) / 32u;
-    uint32_t carry = before;
-    for (uint32_t base = g0; base < g1; base += kPassThreads) {
-        // exclusive scan of this tile's group counts
-        const uint32_t g = base + threadIdx.x;
-        const uint32_t c = g < g1 ? counts[g] : 0u;
-        uint32_t x = c;
+    seg[threadIdx.x] = 0u;
+    if (threadIdx.x == 0) s_t0 = *top;
+    // what the warp needs of its next group, loaded ahead: the group's count and
+    // bitmap words, and this lane's part of the counts from the segment's start
+    // (added where they are used, so nothing waits here while a segment is 64 groups)
+    uint32_t cnt = 0, part0 = 0, part1 = 0, myword = 0;
+    auto load_group = [&](uint32_t g) {
+        cnt = part0 = part1 = myword = 0;
+        if (g >= ng) return;
+        cnt = counts[g];
+        const uint32_t k = (g / kSegGroups >> seg_shift << seg_shift) * kSegGroups + lane;
+        if (k < g) part0 = counts[k];
+        if (k + 32u < g) part1 = counts[k + 32u];
+        for (uint32_t m = k + 64u; m < g; m += 32u) part0 += counts[m];
+        const uint32_t wi = g * (kGroupIds / 32) + (lane & 7u);
+        if (lane < 8u && wi < nwords) myword = bits[wi];
+    };
+    load_group(blockIdx.x * kWarps + wid);
+    __syncthreads();
+    // the segments' counts: 16 lanes read 64 groups (counts is 16-byte aligned, a device allocation)
+    for (uint32_t q = threadIdx.x; q < (ng + kSegGroups - 1) / kSegGroups * 16u; q += kPassThreads) {
+        const uint32_t g = 4u * q;
+        uint32_t c = 0;
+        if (g + 4u <= ng) {
+            const uint4 c4 = reinterpret_cast<const uint4*>(counts)[q];
+            c = c4.x + c4.y + c4.z + c4.w;
+        } else {
+            for (uint32_t k = g; k < ng; ++k) c += counts[k];
+        }
+        // (the bound on q is a multiple of 16, so the 16 lanes of a segment leave the loop together)
+        const uint32_t half = 0xffffu << (lane & 16u);
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) c += __shfl_xor_sync(half, c, o);
+        if ((lane & 15u) == 0 && c) atomicAdd(&seg[(q / 16u) >> seg_shift], c);
+    }
+    __syncthreads();
+    uint32_t total_u = 0;
+    {
+        const uint32_t mine = seg[threadIdx.x];
+        uint32_t x = mine;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
             if (lane >= (uint32_t)o) x += y;
         }
-        __syncthreads();   // red is free again
-        if (lane == 31) red[0][wid] = x;
+        if (lane == 31) red[wid] = x;
         __syncthreads();
-        uint32_t wpre = 0;
-        for (uint32_t k = 0; k < wid; ++k) wpre += red[0][k];
-        excl[threadIdx.x] = carry + wpre + x - c;
-        uint32_t tile_total = 0;
-        for (int k = 0; k < kWarps; ++k) tile_total += red[0][k];
-        __syncthreads();
-        // one warp per group with members
-        const uint32_t tn = min(g1 - base, (uint32_t)kPassThreads);
-        for (uint32_t t = wid; t < tn; t += kWarps) {
-            const uint32_t gg = base + t;
-            const uint32_t r0 = excl[t];
-            const uint32_t cnt = (t + 1 < tn ? excl[t + 1] : carry + tile_total) - r0;
-            if (cnt == 0) continue;                                    // warp-uniform
-            if (mode == 0 && (int32_t)r0 >= applied) continue;         // no slot left for this group
-            const uint32_t wi = gg * (kGroupIds / 32) + (lane & 7u);
-            const uint32_t myword = lane < 8u && wi < nwords ? bits[wi] : 0u;
-            // lane l takes bit l of each of the 8 words; every load and store of
-            // the group is independent of the others, so all are in flight at once
-            uint32_t r = r0;
-            uint32_t slot[kGroupIds / 32];
-#pragma unroll
-            for (uint32_t j = 0; j < kGroupIds / 32; ++j) {
-                const uint32_t word = __shfl_sync(0xffffffffu, myword, j);
-                const bool bit = (word >> lane) & 1u;
-                const uint32_t rr = r + __popc(word & ((1u << lane) - 1u));
-                const uint32_t id = gg * kGroupIds + j * 32u + lane;
-                slot[j] = kNoSlot;
-                if (bit && id < nbits) {
-                    if (mode == 0) {
-                        const int32_t fi = t0 - 1 - (int32_t)rr;
-                        // free-list state uploaded by a caller may be inconsistent: never index outside the pool
-                        if ((int32_t)rr < applied && fi >= 0 && (uint32_t)fi < M) slot[j] = free_list[fi];
-                    } else {
-                        const int32_t fi = t0 + (int32_t)rr;
-                        if (fi >= 0 && (uint32_t)fi < M) free_list[fi] = id;
-                    }
-                }
-                r += __popc(word);
-            }
-            if (mode == 0) {
-                // 48-byte records as three 16-byte words (device allocations and
-                // 48-byte strides keep every record 16-byte aligned); kBatch records'
-                // loads are issued before their stores
-                constexpr uint32_t kBatch = 2;
-                static_assert(sizeof(mpm_diffuse_particle) == 48, "three 16-byte words per record");
-#pragma unroll
-                for (uint32_t jb = 0; jb < kGroupIds / 32; jb += kBatch) {
-                    uint4 rec[kBatch][3];
-#pragma unroll
-                    for (uint32_t q = 0; q < kBatch; ++q) {
-                        if (slot[jb + q] < M) {
-                            const uint4* src =
-                                reinterpret_cast<const uint4*>(staging + gg * kGroupIds + (jb + q) * 32u + lane);
-                            rec[q][0] = src[0];
-                            rec[q][1] = src[1];
-                            rec[q][2] = src[2];
-                        }
-                    }
-#pragma unroll
-                    for (uint32_t q = 0; q < kBatch; ++q) {
-                        if (slot[jb + q] < M) {
-                            const uint32_t sl = slot[jb + q];
-                            uint4* dst = reinterpret_cast<uint4*>(pool + sl);
-                            dst[0] = rec[q][0];
-                            dst[1] = rec[q][1];
-                            dst[2] = rec[q][2];
-                            atomicOr(&alive_mask[sl >> 5], 1u << (sl & 31u));   // staged records are alive
-                        }
-                    }
-                }
-            }
+        uint32_t before = x - mine;
+        for (uint32_t k = 0; k < (uint32_t)kWarps; ++k) {
+            if (k < wid) before += red[k];
+            total_u += red[k];
         }
-        carry += tile_total;
-        __syncthreads();   // excl is rewritten by the next tile
+        seg[threadIdx.x] = before;
+    }
+    __syncthreads();
+    const int32_t t0 = s_t0, total = (int32_t)total_u;
+    const int32_t applied = mode == 0 ? (t0 > 0 ? (total < t0 ? total : t0) : 0) : total;
+    for (uint32_t gg = blockIdx.x * kWarps + wid; gg < ng; gg += gridDim.x * kWarps) {
+        const uint32_t sg = gg / kSegGroups >> seg_shift;
+        if (mode == 0 && (int32_t)seg[sg] >= applied) break;   // no slot left for this group or any after it
+        // the count before the group: its segment's and that of the groups between
+        const uint32_t r0 = __reduce_add_sync(0xffffffffu, part0 + part1) + seg[sg];
+        const uint32_t members = cnt, words = myword;
+        load_group(gg + gridDim.x * kWarps);
+        if (members == 0) continue;                            // warp-uniform
+        if (mode == 0 && (int32_t)r0 >= applied) break;
+        // lane l takes bit l of each of the 8 words
+        uint32_t r = 0;
+#pragma unroll
+        for (uint32_t j = 0; j < kGroupIds / 32; ++j) {
+            const uint32_t word = __shfl_sync(0xffffffffu, words, j);
+            const uint32_t rr = r + __popc(word & ((1u << lane) - 1u));
+            if ((word >> lane) & 1u) {
+                if (mode == 0) {
+                    member[wid][rr] = (uint8_t)(j * 32u + lane);
+                } else {
+                    const uint32_t id = gg * kGroupIds + j * 32u + lane;
+                    const int32_t fi = t0 + (int32_t)(r0 + rr);
+                    if (id < nbits && fi >= 0 && (uint32_t)fi < M) free_list[fi] = id;
+                }
+            }
+            r += __popc(word);
+        }
+        if (mode == 0) {
+            // the group's spawners side by side: a lane's slot and its record
+            // (48 bytes as three 16-byte words: device allocations and 48-byte
+            // strides keep every record 16-byte aligned) are loaded at once
+            static_assert(sizeof(mpm_diffuse_particle) == 48, "three 16-byte words per record");
+            __syncwarp();
+            const uint32_t here = min(min(members, r), (uint32_t)(applied - (int32_t)r0));
+            for (uint32_t q = lane; q < here; q += 32u) {
+                const uint32_t id = gg * kGroupIds + member[wid][q];
+                const int32_t fi = t0 - 1 - (int32_t)(r0 + q);
+                // free-list state uploaded by a caller may be inconsistent: never index outside the pool
+                if (id >= nbits || fi < 0 || (uint32_t)fi >= M) continue;
+                const uint32_t sl = free_list[fi];
+                const uint4* src = reinterpret_cast<const uint4*>(staging + id);
+                const uint4 a = src[0], b = src[1], c = src[2];
+                if (sl < M) {
+                    uint4* dst = reinterpret_cast<uint4*>(pool + sl);
+                    dst[0] = a;
+                    dst[1] = b;
+                    dst[2] = c;
+                    atomicOr(&alive_mask[sl >> 5], 1u << (sl & 31u));   // staged records are alive
+                }
+            }
+            __syncwarp();   // member is rewritten by the next group
+        }
     }
     // (kill pass) the spawn bits and counts were last read by the spawn pass:
     // clear them for the next substep's G2P
@@ -794,13 +845,12 @@ __global__ void __launch_bounds__(kPassThreads, 2) k_freelist_pass(const uint32_
     }
 }
 
-// Blocks of one free-list pass over ng groups: about one group per warp, at
-// most two blocks per SM's worth.
-static inline void freelist_grid(uint32_t ng, uint32_t& B, uint32_t& R) {
+// Blocks of one free-list pass over ng groups (about one group per warp, at
+// most two blocks per SM's worth) and the groups of a segment, 64 << shift.
+static inline void freelist_grid(uint32_t ng, uint32_t& B, uint32_t& shift) {
     constexpr uint32_t kWarps = kPassThreads / 32, kMaxBlocks = 2 * 148;
     B = std::max(1u, std::min(blocks_for(ng, kWarps), kMaxBlocks));
-    R = std::max(1u, blocks_for(ng, B));
-    B = std::max(1u, blocks_for(ng, R));
+    for (shift = 0; ((blocks_for(ng, kSegGroups) + (1u << shift) - 1) >> shift) > kMaxSegs;) ++shift;
 }
 
 cudaError_t launch_alive_mask_build(Scene& s) {
@@ -838,9 +888,9 @@ cudaError_t launch_diffuse(Scene& s, bool eval, const mpm_params* P_dev, const m
             s.launches++;
         }
         // (the binned engine's G2P has already counted the spawners per group)
-        uint32_t B, R;
-        freelist_grid(ng, B, R);
-        k_freelist_pass<<<B, kPassThreads, 0, st>>>(d.spawn_bits, n, d.block_counts, ng, R, d.top, d.rank_state,
+        uint32_t B, shift;
+        freelist_grid(ng, B, shift);
+        k_freelist_pass<<<B, kPassThreads, 0, st>>>(d.spawn_bits, n, d.block_counts, ng, shift, d.top, d.rank_state,
                                                     d.free_list, d.staging, d.pool, d.max_count, 0, nullptr, nullptr, 0,
                                                     nullptr, 0, d.alive_mask);
         s.launches += 1;
@@ -859,9 +909,9 @@ cudaError_t launch_diffuse(Scene& s, bool eval, const mpm_params* P_dev, const m
         else
             k_diffuse_advect<<<mg, kThreads, 0, st>>>(d.pool, s.mvf, s.vel4, P, adv, s.walls, d.kill_bits,
                                                       d.kill_counts, d.alive_mask);
-        uint32_t B, R;
-        freelist_grid(mg, B, R);
-        k_freelist_pass<<<B, kPassThreads, 0, st>>>(d.kill_bits, M, d.kill_counts, mg, R, d.top, d.rank_state,
+        uint32_t B, shift;
+        freelist_grid(mg, B, shift);
+        k_freelist_pass<<<B, kPassThreads, 0, st>>>(d.kill_bits, M, d.kill_counts, mg, shift, d.top, d.rank_state,
                                                     d.free_list, nullptr, d.pool, M, 1, d.top_hist, d.spawn_bits,
                                                     (n + 31u) / 32u, d.block_counts, ng, nullptr);
         s.launches += 2;
