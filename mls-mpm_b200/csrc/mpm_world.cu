@@ -2,9 +2,10 @@
 //
 // Same arithmetic as mpm_kernels.cu (and so the same bits), organised for
 // the B200:
-//   * Particles are sorted by (tile, cell) every substep (counting sort: the
-//     rank of each particle in its new cell is taken in G2P, then a scan per
-//     16x8x8-cell tile and a two-level scan over tiles) and each tile's
+//   * Particles are sorted by (tile, cell) every substep (counting sort: G2P
+//     takes the rank of each particle in its new cell and counts each
+//     16x8x8-cell tile's particles, so that one launch can scan the tiles and
+//     the cells inside them and a second places the particles) and each tile's
 //     particles are cut into chunks of up to kChunk consecutive particles
 //     (kChunkSmall in worlds too small to fill the chunk kernels' grid).
 //     The new layout reads the previous one through a permutation (new
@@ -21,7 +22,7 @@
 //     out through template indices.  Particles whose stencil leaves the halo
 //     or the grid take a direct path with the reference's own indexing.
 //   * Latency hiding: each block keeps its chunk's scene descriptor in shared
-//     memory, loads the next chunk's header (packed by P2G_MASS) a chunk
+//     memory, loads the next chunk's header (packed by the binning) a chunk
 //     ahead, and P2G_MOM copies the next chunk's halo masses (cp.async) and
 //     loads its first particle while the current chunk runs.
 //   * Scenes: cells, tiles and particle ids of every scene are ranges of the
@@ -38,7 +39,8 @@
 //     this substep's density), staging records by particle id; G2P also
 //     counts the spawners per group of ids for the free-list ranking.
 //   * A substep (diffuse update included) is captured once per layout parity
-//     as a CUDA graph and replayed.
+//     as a CUDA graph and replayed, once the same arguments have run a few
+//     times eagerly.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -109,9 +111,7 @@ WorldView World::view() const {
     v.cell_count = cell_count; v.cell_start = cell_start;
     v.key = key; v.rank = rank; v.perm = perm;
     v.tile_flags = tile_flags; v.tile_cnt = tile_cnt; v.tile_base = tile_base;
-    v.par = (uint32_t)cur;
-    v.chunk_hdr = chunk_hdr[cur];
-    v.chunk_hdr_prev = chunk_hdr[cur ^ 1];
+    v.chunk_hdr = chunk_hdr;
     v.tile_occ_list = tile_occ_list; v.tile_grid_list = tile_grid_list;
     v.ctrl = ctrl; v.dens = dens;
     v.health = health;
@@ -344,8 +344,8 @@ __global__ void __launch_bounds__(1024) k_tiles_list(WorldView v) {
     }
     if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
         v.ctrl->n_occ = n0 + n;
-        v.ctrl->cursor[v.par] = (uint32_t)((sum0 + sum) >> 32);
-        v.ctrl->chunks[v.par] = (uint32_t)(sum0 + sum);
+        v.ctrl->n_pos = (uint32_t)((sum0 + sum) >> 32);
+        v.ctrl->n_chunks = (uint32_t)(sum0 + sum);
     }
 }
 
@@ -478,8 +478,8 @@ __global__ void __launch_bounds__(kTileCells) k_bin_cells(WorldView v) {
             all += sum;
         }
         if (blockIdx.x == 0 && threadIdx.x == 0) {
-            v.ctrl->cursor[v.par] = (uint32_t)(all >> 32);
-            v.ctrl->chunks[v.par] = (uint32_t)all;
+            v.ctrl->n_pos = (uint32_t)(all >> 32);
+            v.ctrl->n_chunks = (uint32_t)all;
         }
         __syncthreads();
     }
@@ -662,8 +662,8 @@ __device__ __forceinline__ float2 sadd(float2 a, float2 b) { return make_float2(
 // Chunks in shared memory
 // ---------------------------------------------------------------------------
 // Chunks of the layout of parity p.
-__device__ __forceinline__ uint32_t chunk_count(const WorldView& v, uint32_t p) {
-    return min(v.ctrl->chunks[p], v.chunk_cap);
+__device__ __forceinline__ uint32_t chunk_count(const WorldView& v) {
+    return min(v.ctrl->n_chunks, v.chunk_cap);
 }
 
 // Lane order of the P2G chunk kernels: lane l of warp w has offset 8*l + w
@@ -814,7 +814,7 @@ __global__ void __launch_bounds__(kChunkThreads) k_p2g_mass_chunks(WorldView v, 
                                                                    int32_t* __restrict__ cm) {
     constexpr int kPer = kC / kChunkThreads;
     __shared__ int32_t acc[kHaloCells];
-    const uint32_t nch = chunk_count(v, v.par);
+    const uint32_t nch = chunk_count(v);
     __shared__ ChunkHdr hs;
     __shared__ uint4 nhs[2];                         // the next chunk's header words
     // scene descriptors of this chunk and the next (thread 0 copies the next
@@ -928,7 +928,7 @@ __device__ __forceinline__ const SceneDesc* tile_cell(const WorldView& v, uint32
 __global__ void __launch_bounds__(256) k_decode_tiles(WorldView v, const int32_t* __restrict__ cm,
                                                       float* __restrict__ cmf) {
     // the binning is done: the layout's size for the passes between substeps
-    if (blockIdx.x == 0 && threadIdx.x == 0) v.ctrl->total_pos = min(v.ctrl->cursor[v.par], v.npos);
+    if (blockIdx.x == 0 && threadIdx.x == 0) v.ctrl->total_pos = min(v.ctrl->n_pos, v.npos);
     const uint32_t total = v.ctrl->n_grid * kTileCells;
     for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x) {
         uint32_t c;
@@ -1413,7 +1413,7 @@ __global__ void __launch_bounds__(kChunkThreads, MPM_MOM_MINB) k_p2g_mom_chunks(
     // the scene descriptors of the current chunk and of the next one, which is
     // copied while the current chunk runs (no wait when the scene changes)
     __shared__ SceneDesc ssd[2];
-    const uint32_t nch = chunk_count(v, v.par);
+    const uint32_t nch = chunk_count(v);
     const uint32_t G = gridDim.x;
     if (blockIdx.x >= nch) return;   // block-uniform
     const size_t plane = v.npos;
@@ -1870,7 +1870,7 @@ __global__ void __launch_bounds__(kChunkThreads, MPM_G2P_MINB) k_g2p_chunks(Worl
     constexpr int kPer = kC / kChunkThreads;
     __shared__ float4 vh[kHaloCells];   // staged grid velocities (x, y, z, 0)
     __shared__ uint4 nhs[2];              // the next chunk's header words
-    const uint32_t nch = chunk_count(v, v.par);
+    const uint32_t nch = chunk_count(v);
     const size_t plane = v.npos;
     __shared__ ChunkHdr hs;
     // scene descriptors of this chunk and the next (thread 0 copies the next
@@ -2065,8 +2065,7 @@ template <class F> static void world_arrays(World& w, F&& f) {
     f(w.tile_flags, T * 4);
     f(w.tile_cnt, T * 4);
     f(w.tile_base, T * 8);
-    f(w.chunk_hdr[0], (size_t)w.chunk_cap * 32);
-    f(w.chunk_hdr[1], (size_t)w.chunk_cap * 32);
+    f(w.chunk_hdr, (size_t)w.chunk_cap * 32);
     f(w.tile_occ_list, T * 4);
     f(w.tile_grid_list, T * 4);
     f(w.tile_scene, T * 4);

@@ -64,17 +64,15 @@ struct Ctrl {
     uint32_t n_occ;             // occupied tiles listed for the binning (worlds of many tiles)
     uint32_t n_grid;            // grid tiles of this substep (cleared by G2P, after their last use)
     uint32_t total_pos;         // positions of the layout, holes of removed scenes included
-    uint32_t pad;
-    // by substep parity, written by the binning
-    uint32_t cursor[2];         // positions of the layout
-    uint32_t chunks[2];         // chunks of the layout
+    // written by the binning
+    uint32_t n_pos;             // positions of the layout
+    uint32_t n_chunks;          // chunks of the layout
 };
 
 // Everything the device kernels need (passed by value).
 struct WorldView {
     uint32_t npos;             // capacity of the position space
     uint32_t ntiles;           // tiles in use (end of the allocated tile range)
-    uint32_t par;              // this substep's parity
     uint32_t chunk_cap;        // capacity of the chunk list
     uint32_t chunk;            // particles per chunk this substep (kChunk or kChunkSmall)
     const SceneDesc* scenes;
@@ -86,7 +84,6 @@ struct WorldView {
     uint32_t* perm;            // npos: position -> position of the previous layout
     uint32_t* tile_flags;      // per tile
     uint4* chunk_hdr;          // per chunk of this substep's layout, 2 words: the packed ChunkHdr (written by the binning)
-    const uint4* chunk_hdr_prev;   // the previous layout's
     uint32_t* tile_cnt;        // per tile: particles for the next binning (counted by G2P and imports)
     uint2* tile_base;          // per listed tile: its first position and chunk (worlds of many tiles)
     uint32_t* tile_occ_list;
@@ -108,8 +105,8 @@ struct DiffuseView {
 
 // Reference-layout particle buffers (by particle id) that the substep keeps
 // current for the one scene of a single-scene world whose consumer reads them
-// every frame (a renderer's vertex inputs): G2P writes pos/vel, P2G_MOM
-// writes density.  Disabled: nothing written.
+// every frame (a renderer's vertex inputs): G2P writes position, velocity and
+// density, or k_mirror after it.  Disabled: nothing written.
 struct RefOut {
     int enabled;
     uint32_t scene;
@@ -204,7 +201,7 @@ struct World {
     uint32_t* tile_flags = nullptr;
     uint32_t* tile_cnt = nullptr;
     uint2* tile_base = nullptr;
-    uint4* chunk_hdr[2] = {nullptr, nullptr};   // by parity
+    uint4* chunk_hdr = nullptr;
     uint32_t chunk_cap = 0;
     uint32_t chunk = kChunk;   // chunk size of the substep being enqueued
     uint32_t* tile_occ_list = nullptr;
