@@ -306,7 +306,7 @@ mpm_status mpm_compact_noalloc(const mpm_ray_params* del, uint32_t n, const floa
 typedef enum mpm_phase {
     MPM_PHASE_CLEAR = 0,        /* CLEAR (shaders.js:196-210)                */
     MPM_PHASE_P2G_MASS = 1,     /* COMPUTE_WEIGHTS + P2G_MASS (216-274)      */
-    MPM_PHASE_DECODE_MASS = 2,  /* DECODE_MASS (373-384)                     */
+    MPM_PHASE_DECODE_MASS = 2,  /* DECODE_MASS (373-384); inside P2G_MOM and UPDATE_GRID in small worlds */
     MPM_PHASE_P2G_MOM = 3,      /* P2G_MOM (276-371)                         */
     MPM_PHASE_UPDATE_GRID = 4,  /* UPDATE_GRID (435-513)                     */
     MPM_PHASE_APPLY_HAND = 5,   /* APPLY_HAND (394-433)                      */

@@ -814,6 +814,8 @@ __global__ void __launch_bounds__(kChunkThreads) k_p2g_mass_chunks(WorldView v, 
                                                                    int32_t* __restrict__ cm) {
     constexpr int kPer = kC / kChunkThreads;
     __shared__ int32_t acc[kHaloCells];
+    // the binning is done: the layout's size for the passes between substeps
+    if (blockIdx.x == 0 && threadIdx.x == 0) v.ctrl->total_pos = min(v.ctrl->n_pos, v.npos);
     const uint32_t nch = chunk_count(v);
     __shared__ ChunkHdr hs;
     __shared__ uint4 nhs[2];                         // the next chunk's header words
@@ -927,8 +929,6 @@ __device__ __forceinline__ const SceneDesc* tile_cell(const WorldView& v, uint32
 
 __global__ void __launch_bounds__(256) k_decode_tiles(WorldView v, const int32_t* __restrict__ cm,
                                                       float* __restrict__ cmf) {
-    // the binning is done: the layout's size for the passes between substeps
-    if (blockIdx.x == 0 && threadIdx.x == 0) v.ctrl->total_pos = min(v.ctrl->n_pos, v.npos);
     const uint32_t total = v.ctrl->n_grid * kTileCells;
     for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x) {
         uint32_t c;
@@ -1002,8 +1002,9 @@ __device__ __forceinline__ void hand_push(const mpm_hand_params& H, int32_t cx, 
 }
 
 __global__ void __launch_bounds__(256) k_update_tiles(WorldView v, const int32_t* __restrict__ cm,
-                                                      const int32_t* __restrict__ mv, float* __restrict__ mvf,
-                                                      float4* __restrict__ vel4, int32_t* __restrict__ cm_next,
+                                                      const int32_t* __restrict__ mv, float* __restrict__ cmf,
+                                                      float* __restrict__ mvf, float4* __restrict__ vel4,
+                                                      int32_t* __restrict__ cm_next,
                                                       int32_t* __restrict__ mv_next) {
     const uint32_t total = v.ctrl->n_grid * kTileCells;
     for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x) {
@@ -1015,6 +1016,7 @@ __global__ void __launch_bounds__(256) k_update_tiles(WorldView v, const int32_t
         cm_next[idx] = 0;
         mv_next[3 * (size_t)idx + 0] = 0; mv_next[3 * (size_t)idx + 1] = 0; mv_next[3 * (size_t)idx + 2] = 0;
         const float c = decode(cm[idx]);
+        if (cmf) cmf[idx] = c;   // (given when no DECODE_MASS pass ran)
         float* out = mvf + 3 * (size_t)idx;
         float vx = 0.0f, vy = 0.0f, vz = 0.0f;
         if (c > 0.0f) update_cell(sd, cm, mv, idx, c, cx, cy, cz, vx, vy, vz);
@@ -1288,7 +1290,9 @@ __device__ __forceinline__ float density_shared(const PW& w, const float* m) {
     return d;
 }
 
-// P2G_MOM for one particle whose inputs are loaded.
+// P2G_MOM for one particle whose inputs are loaded.  kRaw: scmf holds the i32
+// masses (P2G_MASS's sums) instead of the decoded ones.
+template <bool kRaw>
 __device__ __forceinline__ void mom_particle(const WorldView& v, const ChunkHdr& h, const SceneDesc& sd, bool valid,
                                              const float4 pm, const float4 r0, const float4 r1, const float4 r2,
                                              const float* mh, int32_t (*acc)[kHaloCells],
@@ -1308,7 +1312,8 @@ __device__ __forceinline__ void mom_particle(const WorldView& v, const ChunkHdr&
             for (int jj = 0; jj < 3; ++jj)
                 for (int i = 0; i < 3; ++i) {
                     const uint32_t cidx = baseIdx + (uint32_t)k * SLICE + (uint32_t)jj * X + (uint32_t)i;
-                    const float cmass = cidx < G ? scmf[cidx] : 0.0f;
+                    float cmass = cidx < G ? scmf[cidx] : 0.0f;
+                    if (kRaw) cmass = decode(__float_as_int(cmass));
                     density += w.wx[i] * w.wy[jj] * w.wz[k] * cmass;
                 }
     }
@@ -1375,11 +1380,23 @@ __device__ __forceinline__ void mom_particle(const WorldView& v, const ChunkHdr&
 // the halo masses of the block's next chunk are copied into the other
 // staging buffer (cp.async) and its first particle's inputs are loaded; the
 // accumulators are zeroed by the flush that reads them.
+//
+// kRaw (world_substep's rule: worlds of about one small chunk a block, whose
+// substep costs its launches, not its work): no DECODE_MASS pass; cmf points to
+// the i32 masses, each thread decodes what it staged, and UPDATE_GRID, which
+// decodes every cell anyway, writes the decoded grid.
 __device__ __forceinline__ void stage_masses_async(const WorldView& v, const ChunkHdr& hh,
                                                    const float* __restrict__ cmf, float* buf) {
     const GridDims g = grid_dims(v.scenes[hh.scene]);
     const float* src = cmf + g.cell_base;
     halo_columns<kChunkThreads>(hh, g, [&](int s, uint32_t cell) { cp_async4z(buf + s, src + cell, 4u); });
+}
+// Decodes the i32 masses that this thread staged, once its copies have landed.
+__device__ __forceinline__ void decode_staged(const WorldView& v, const ChunkHdr& hh, float* buf) {
+    halo_columns<kChunkThreads>(hh, grid_dims(v.scenes[hh.scene]), [&](int s, uint32_t) {
+        const int32_t m = __float_as_int(buf[s]);
+        if (m != 0) buf[s] = decode(m);   // (the word 0 is 0.0f already)
+    });
 }
 
 // One particle's inputs: four 16-byte words.  A warp's lanes spread over the
@@ -1400,7 +1417,7 @@ __device__ __forceinline__ void mom_load(const WorldView& v, uint32_t p, bool va
     in.row[2] = rows[2 * plane + slot];
 }
 
-template <uint32_t kC>
+template <uint32_t kC, bool kRaw = false>
 __global__ void __launch_bounds__(kChunkThreads, MPM_MOM_MINB) k_p2g_mom_chunks(WorldView v, const float4* __restrict__ posm,
                                                                    const float4* __restrict__ rows,
                                                                    const float* __restrict__ cmf,
@@ -1438,6 +1455,7 @@ __global__ void __launch_bounds__(kChunkThreads, MPM_MOM_MINB) k_p2g_mom_chunks(
     MomLoad in{};
     mom_load(v, p, valid, posm, rows, plane, in);
     cp_async_wait();
+    if (kRaw) decode_staged(v, hdr[0], mh[0]);
     __syncthreads();
     int b = 0;
     for (uint32_t ch = blockIdx.x; ch < nch; ch += G) {
@@ -1476,7 +1494,7 @@ __global__ void __launch_bounds__(kChunkThreads, MPM_MOM_MINB) k_p2g_mom_chunks(
             }
             MomLoad next{};
             mom_load(v, pn, vn, posm, rows, plane, next);
-            mom_particle(v, h, sd, valid, in.pm, in.row[0], in.row[1], in.row[2], mh[b], acc, scmf, smv, dens + p,
+            mom_particle<kRaw>(v, h, sd, valid, in.pm, in.row[0], in.row[1], in.row[2], mh[b], acc, scmf, smv, dens + p,
                          v.health + h.scene);
             p = pn;
             valid = vn;
@@ -1497,6 +1515,7 @@ __global__ void __launch_bounds__(kChunkThreads, MPM_MOM_MINB) k_p2g_mom_chunks(
             atomicAdd(d + 2, a2);
         });
         cp_async_wait();
+        if (kRaw && has_next) decode_staged(v, hdr[b ^ 1], mh[b ^ 1]);
         __syncthreads();
         b ^= 1;
         const uint32_t t = ss_cur;
@@ -2497,14 +2516,21 @@ static cudaError_t enqueue_substep(World& w, Scene* ds, const RefOut& ro, bool t
             k_p2g_mass_chunks<kChunk><<<w.item_blocks, kChunkThreads, 0, st>>>(v, w.posm[cur], cm);
         w.launches++;
     }
-    {
+    // A launch less is worth more than decoding every staged halo until blocks
+    // take a second chunk: frame of 8k particles 13.6 -> 12.7 us, 64k 20.2 -> 19.0
+    // (three scenes in turn), but 230k 56.9 -> 58.8.
+    const bool raw_mass = w.chunk == kChunkSmall && w.n_total <= w.item_blocks * kChunkSmall;
+    if (!raw_mass) {
         Phase ph(prof, MPM_PHASE_DECODE_MASS);
         k_decode_tiles<<<w.grid_blocks, 256, 0, st>>>(v, cm, w.cmf);
         w.launches++;
     }
     {
         Phase ph(prof, MPM_PHASE_P2G_MOM);
-        if (w.chunk == kChunkSmall)
+        if (raw_mass)
+            k_p2g_mom_chunks<kChunkSmall, true><<<w.item_blocks, kChunkThreads, 0, st>>>(
+                v, w.posm[cur], w.rows[cur], reinterpret_cast<const float*>(cm), mv, w.dens);
+        else if (w.chunk == kChunkSmall)
             k_p2g_mom_chunks<kChunkSmall><<<w.item_blocks, kChunkThreads, 0, st>>>(v, w.posm[cur], w.rows[cur], w.cmf, mv,
                                                                                  w.dens);
         else
@@ -2520,7 +2546,7 @@ static cudaError_t enqueue_substep(World& w, Scene* ds, const RefOut& ro, bool t
     }
     {
         Phase ph(prof, MPM_PHASE_UPDATE_GRID);   // includes APPLY_HAND
-        k_update_tiles<<<w.grid_blocks, 256, 0, st>>>(v, cm, mv, w.mvf, w.vel4, cm_n, mv_n);
+        k_update_tiles<<<w.grid_blocks, 256, 0, st>>>(v, cm, mv, raw_mass ? w.cmf : nullptr, w.mvf, w.vel4, cm_n, mv_n);
         w.launches++;
     }
     // (the spawn bits and group counts G2P adds to were cleared by the
