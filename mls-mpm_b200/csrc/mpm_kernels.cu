@@ -20,6 +20,7 @@
 
 #include "mpm_device.cuh"
 #include "mpm_kernels.h"
+#include "mpm_stencil.h"
 
 namespace mpm {
 
@@ -465,7 +466,7 @@ __device__ __forceinline__ f3 sample_grid_velocity(const float* __restrict__ mvf
     qweights(fy, wy[0], wy[1], wy[2]);
     qweights(fz, wz[0], wz[1], wz[2]);
     f3 v = mk(0.0f, 0.0f, 0.0f);
-    if (vel4 && cx >= 1 && cy >= 1 && cz >= 1 && cx + 1 < X && cy + 1 < Y && cz + 1 < Z) {
+    if (vel4 && stencil_in(cx, 0, X) && stencil_in(cy, 0, Y) && stencil_in(cz, 0, Z)) {
         // the whole stencil lies in the grid: a plane's nine loads are issued
         // before the first is used, at offsets from one cell
         const float4* c0 = vel4 + ((uint32_t)(cz - 1) * (uint32_t)Y + (uint32_t)(cy - 1)) * (uint32_t)X + (uint32_t)(cx - 1);
@@ -490,13 +491,13 @@ __device__ __forceinline__ f3 sample_grid_velocity(const float* __restrict__ mvf
     }
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        const int32_t zz = cz - 1 + k;
+        const int32_t zz = stencil_cell(cz, k);
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
-            const int32_t yy = cy - 1 + j;
+            const int32_t yy = stencil_cell(cy, j);
 #pragma unroll
             for (int i = 0; i < 3; ++i) {
-                const int32_t xx = cx - 1 + i;
+                const int32_t xx = stencil_cell(cx, i);
                 if (xx < 0 || xx >= X || yy < 0 || yy >= Y || zz < 0 || zz >= Z) continue;
                 const uint32_t idx = (uint32_t)((zz * Y + yy) * X + xx);
                 const float w = wx[i] * wy[j] * wz[k];

@@ -51,6 +51,7 @@
 #include "mpm_device.cuh"
 #include "mpm_kernels.h"
 #include "mpm_scene.h"
+#include "mpm_stencil.h"
 #include "mpm_world.h"
 
 // MPM_MIRROR_KEEP (default): the render mirrors' stores carry an L2
@@ -610,6 +611,12 @@ __device__ __forceinline__ PW particle_weights(float px, float py, float pz) {
     return w;
 }
 
+// The reference's linear index of the stencil's first cell (shaders.js:303-304
+// and 598-599), which wraps for cells outside the grid.
+__device__ __forceinline__ uint32_t stencil_base(const PW& w, uint32_t X, uint32_t Y) {
+    return (((uint32_t)w.cz - 1u) * Y + ((uint32_t)w.cy - 1u)) * X + ((uint32_t)w.cx - 1u);
+}
+
 // encode() without the clamp, for values already known to lie in +-20000.
 __device__ __forceinline__ int32_t encode_unclamped(float v) { return __float2int_rz(v * kFixed); }
 
@@ -736,9 +743,8 @@ __device__ __forceinline__ void copy_scene_async_one(const WorldView& v, uint32_
 // the grid (then shared-memory accumulation / gathering is exact); otherwise
 // the particle takes the direct path with the reference's indexing.
 __device__ __forceinline__ bool in_halo(int32_t cx, int32_t cy, int32_t cz, const ChunkHdr& h, const SceneDesc& sd) {
-    return cx - 1 >= h.ox && cy - 1 >= h.oy && cz - 1 >= h.oz && cx + 1 < h.ox + h.hx && cy + 1 < h.oy + h.hy &&
-           cz + 1 < h.oz + h.hz && cx >= 1 && cy >= 1 && cz >= 1 && cx + 1 < (int32_t)sd.X &&
-           cy + 1 < (int32_t)sd.Y && cz + 1 < (int32_t)sd.Z;
+    return stencil_in(cx, h.ox, h.hx) && stencil_in(cy, h.oy, h.hy) && stencil_in(cz, h.oz, h.hz) &&
+           stencil_in(cx, 0, (int32_t)sd.X) && stencil_in(cy, 0, (int32_t)sd.Y) && stencil_in(cz, 0, (int32_t)sd.Z);
 }
 __device__ __forceinline__ bool in_halo(const PW& w, const ChunkHdr& h, const SceneDesc& sd) {
     return in_halo(w.cx, w.cy, w.cz, h, sd);
@@ -873,7 +879,7 @@ __global__ void __launch_bounds__(kChunkThreads) k_p2g_mass_chunks(WorldView v, 
                 for (int kk = 0; kk < 3; ++kk)
                     for (int j = 0; j < 3; ++j)
                         for (int i = 0; i < 3; ++i) {
-                            const int32_t xx = w.cx - 1 + i, yy = w.cy - 1 + j, zz = w.cz - 1 + kk;
+                            const int32_t xx = stencil_cell(w.cx, i), yy = stencil_cell(w.cy, j), zz = stencil_cell(w.cz, kk);
                             if (xx < 0 || xx >= X || yy < 0 || yy >= Y || zz < 0 || zz >= Z) continue;
                             const float ww = w.wx[i] * w.wy[j] * w.wz[kk];
                             const int32_t e = encode(ww * q[r].w);
@@ -1302,7 +1308,7 @@ __device__ __forceinline__ void mom_particle(const WorldView& v, const ChunkHdr&
     const PW w = particle_weights(pm.x, pm.y, pm.z);
     const bool fast = valid && in_halo(w, h, sd);
     const int hb = halo_base(h, w.cx, w.cy, w.cz);
-    const uint32_t baseIdx = (uint32_t)(((w.cz - 1) * (int32_t)sd.Y + (w.cy - 1)) * (int32_t)X + (w.cx - 1));
+    const uint32_t baseIdx = stencil_base(w, X, sd.Y);
     // density (shaders.js:305-313), k, j, i order
     float density = 0.0f;
     if (fast) {
@@ -1686,17 +1692,16 @@ __device__ MPM_G2P_RARE G2PSum g2p_gather_direct(const PW w, const float4 q, con
 #pragma unroll
     for (int e = 0; e < 9; ++e) B[e] = 0.0f;
     const uint32_t SLICE = X * Y;
-    const int32_t bx = w.cx - 1, by = w.cy - 1, bz = w.cz - 1;
-    const uint32_t baseIdx = (uint32_t)((bz * (int32_t)Y + by) * (int32_t)X + bx);
+    const uint32_t baseIdx = stencil_base(w, X, Y);
     for (int k = 0; k < 3; ++k) {
         const float wzk = w.wz[k];
-        const float dzk = __int2float_rn(bz + k) - q.z + 0.5f;
+        const float dzk = __int2float_rn(stencil_cell(w.cz, k)) - q.z + 0.5f;
         for (int jj = 0; jj < 3; ++jj) {
             const float wyzk = w.wy[jj] * wzk;
-            const float dyj = __int2float_rn(by + jj) - q.y + 0.5f;
+            const float dyj = __int2float_rn(stencil_cell(w.cy, jj)) - q.y + 0.5f;
             for (int i = 0; i < 3; ++i) {
                 const float ww = w.wx[i] * wyzk;
-                const float dxi = __int2float_rn(bx + i) - q.x + 0.5f;
+                const float dxi = __int2float_rn(stencil_cell(w.cx, i)) - q.x + 0.5f;
                 const uint32_t cidx = baseIdx + (uint32_t)k * SLICE + (uint32_t)jj * X + (uint32_t)i;
                 float cvx = 0.0f, cvy = 0.0f, cvz = 0.0f;
                 if (cidx < G) {
