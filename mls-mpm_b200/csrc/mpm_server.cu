@@ -339,6 +339,31 @@ mpm_status mpm_server_run(mpm_server* s, mpm_server_stats* stats) {
     }
     std::vector<Job*> active;
     std::deque<Job*> retired;   // their states are on the way to their blocks, or there and not yet moved on
+    // However the run ends, what has retired is finished: the device's queue is
+    // waited for (a few substeps), the kept states are moved on and the blocks go
+    // back to the pool.
+    struct Finish {
+        mpm_server* s;
+        cudaStream_t stream;
+        std::deque<Job*>& retired;
+        const std::vector<Job*>& jobs;
+        bool done = false;
+        cudaError_t run() {
+            done = true;
+            const cudaError_t e = cudaStreamSynchronize(stream);
+            if (e != cudaSuccess) return e;
+            for (Job* j : retired) {
+                collect(*j, j->state_bytes());
+                j->state = 2;
+            }
+            for (Job* j : jobs)
+                if (j->state == 2) s->pool.give(j->block);
+            return e;
+        }
+        ~Finish() {
+            if (!done) run();
+        }
+    } finish{s, stream, retired, this_run};
     uint64_t k = 0, updates = 0, active_sum = 0, active_max = 0;
     const bool keep = (s->flags & MPM_SERVER_KEEP_STATE) != 0;
     s->t0 = Clock::now();
@@ -410,13 +435,7 @@ mpm_status mpm_server_run(mpm_server* s, mpm_server_stats* stats) {
             retired.pop_front();
         }
     }
-    if (cudaStreamSynchronize(stream) != cudaSuccess) return sfail(MPM_ERR_DEVICE, "final sync");
-    for (Job* j : retired) {
-        collect(*j, j->state_bytes());
-        j->state = 2;
-    }
-    for (Job* j : this_run)
-        if (j->state == 2) s->pool.give(j->block);
+    if (finish.run() != cudaSuccess) return sfail(MPM_ERR_DEVICE, "final sync");
     if (stats) {
         std::memset(stats, 0, sizeof *stats);
         std::vector<double> lat;
