@@ -166,6 +166,7 @@ __global__ void k_import(WorldView v, uint32_t scene, uint32_t pos0, const float
     const float4 vv = vel ? vel[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     posm[p] = make_float4(q.x, q.y, q.z, mass[i]);
     ids[p] = sd.id_base + i;
+    v.dens[p] = 0.0f;   // (the position's last density belongs to another particle)
     const float v3[3] = {vv.x, vv.y, vv.z};
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
