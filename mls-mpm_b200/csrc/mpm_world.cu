@@ -111,7 +111,7 @@ WorldView World::view() const {
     v.tile_scene = tile_scene;
     v.cell_count = cell_count; v.cell_start = cell_start;
     v.key = key; v.rank = rank; v.perm = perm;
-    v.tile_flags = tile_flags; v.tile_cnt = tile_cnt; v.tile_base = tile_base;
+    v.tile_flags = tile_flags; v.tile_cnt = tile_cnt; v.tile_base = tile_base; v.tile_group = tile_group;
     v.chunk_hdr = chunk_hdr;
     v.tile_occ_list = tile_occ_list; v.tile_grid_list = tile_grid_list;
     v.ctrl = ctrl; v.dens = dens;
@@ -302,43 +302,56 @@ __device__ __forceinline__ void tile_scan(uint64_t load, TileScan& buf, uint64_t
     n = __shfl_sync(0xffffffffu, wo, 31);
 }
 
-// The occupied tiles in index order with their first position and chunk, for
-// the binning of worlds of more than kScanTiles tiles: one block per 1,024
-// tiles, which adds up the tiles before its own by itself (no block waits for
-// another).
-__global__ void __launch_bounds__(1024) k_tiles_list(WorldView v) {
-    __shared__ TileScan buf[2];
+// A block's sum of a load and a count over its threads, in every thread.
+__device__ __forceinline__ void block_sum_1024(uint64_t& load, uint32_t& n) {
     __shared__ uint64_t part[32];
     __shared__ uint32_t part_n[32];
-    const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
-    uint64_t sum0 = 0;
-    uint32_t n0 = 0;
-    for (uint32_t t = threadIdx.x; t < blockIdx.x * 1024u; t += 1024u) {
-        const uint64_t l = tile_load(v, t);
-        sum0 += l;
-        n0 += l != 0;
-    }
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) {
-        sum0 += __shfl_xor_sync(0xffffffffu, sum0, d);
-        n0 += __shfl_xor_sync(0xffffffffu, n0, d);
+        load += __shfl_xor_sync(0xffffffffu, load, d);
+        n += __shfl_xor_sync(0xffffffffu, n, d);
     }
-    if (lane == 0) {
-        part[wid] = sum0;
-        part_n[wid] = n0;
+    if ((threadIdx.x & 31u) == 0) {
+        part[threadIdx.x >> 5] = load;
+        part_n[threadIdx.x >> 5] = n;
     }
     __syncthreads();
-    sum0 = 0;
-    n0 = 0;
+    load = 0;
+    n = 0;
     for (int k = 0; k < 32; ++k) {
-        sum0 += part[k];
-        n0 += part_n[k];
+        load += part[k];
+        n += part_n[k];
     }
+}
+
+// The load and the number of occupied tiles of each group of 1,024 tiles, for
+// k_tiles_list.
+__global__ void __launch_bounds__(1024) k_tiles_sum(WorldView v) {
+    uint64_t load = tile_load(v, blockIdx.x * 1024u + threadIdx.x);
+    uint32_t n = load != 0;
+    block_sum_1024(load, n);
+    if (threadIdx.x == 0) v.tile_group[blockIdx.x] = make_uint4((uint32_t)load, (uint32_t)(load >> 32), n, 0u);
+}
+
+// The occupied tiles in index order with their first position and chunk, for
+// the binning of worlds of more than kScanTiles tiles: one block per 1,024
+// tiles, which adds up the groups before its own by itself (no block waits for
+// another).
+__global__ void __launch_bounds__(1024) k_tiles_list(WorldView v) {
+    __shared__ TileScan buf;
+    uint64_t sum0 = 0;
+    uint32_t n0 = 0;
+    for (uint32_t g = threadIdx.x; g < blockIdx.x; g += 1024u) {
+        const uint4 q = v.tile_group[g];
+        sum0 += ((uint64_t)q.y << 32) | q.x;
+        n0 += q.z;
+    }
+    block_sum_1024(sum0, n0);
     const uint32_t t = blockIdx.x * 1024u + threadIdx.x;
     const uint64_t load = tile_load(v, t);
     uint64_t pre, sum;
     uint32_t before, n;
-    tile_scan(load, buf[0], pre, before, sum, n);
+    tile_scan(load, buf, pre, before, sum, n);
     if (load != 0) {
         pre += sum0;
         v.tile_occ_list[n0 + before] = t;
@@ -444,13 +457,18 @@ __device__ __forceinline__ ChunkHdr unpack_header(const uint4 a, const uint4 b) 
 //
 // The tiles' first positions come from their particle counts, which G2P keeps:
 // in worlds of up to kScanTiles tiles every block scans the counts itself (one
-// load a thread for 1,024 tiles), in larger ones k_tiles_list does.  A scan of
-// the tile totals found by this kernel took two to five more launches (binning
-// 26 -> 15 us at 8,192 particles, 37 -> 22 us at 1M, 88 -> 72 us at 8M).
+// load a thread for 1,024 tiles), in larger ones k_tiles_sum and k_tiles_list
+// do.  A substep of 1,000 / 100,000 / 2M particles, scanned by the blocks and
+// listed, us: 2,048 tiles 34 48 299 / 37 50 301, 4,000 tiles 37 57 306 / 37 55
+// 306, 5,324 tiles 41 61 314 / 37 55 310, 16,384 tiles 57 88 349 / 37 66 328.
+// (With a list kernel that added up all tiles before its own, not the groups,
+// 131,072 tiles took 49 us for 1,000 particles instead of 37, 698,880 tiles 250
+// instead of 50.)  A scan of the tile totals found by this kernel took two to
+// five more launches (binning 26 -> 15 us at 8,192 particles, 37 -> 22 us at 1M).
 // Handing positions out by one atomic cursor instead puts the tiles of the
 // blocks in flight in any order, which cost 10% of a substep at 8M (the render
 // mirrors' writes by id and the grid's halos then miss L2).
-constexpr uint32_t kScanTiles = 16384;
+constexpr uint32_t kScanTiles = 4096;
 constexpr uint32_t kBinMine = 256;   // tiles of one block in such a world
 __global__ void __launch_bounds__(kTileCells) k_bin_cells(WorldView v) {
     __shared__ uint32_t ws[33];
@@ -2090,6 +2108,7 @@ template <class F> static void world_arrays(World& w, F&& f) {
     f(w.tile_flags, T * 4);
     f(w.tile_cnt, T * 4);
     f(w.tile_base, T * 8);
+    f(w.tile_group, (T + 1023) / 1024 * 16);
     f(w.chunk_hdr, (size_t)w.chunk_cap * 32);
     f(w.tile_occ_list, T * 4);
     f(w.tile_grid_list, T * 4);
@@ -2507,8 +2526,10 @@ static cudaError_t enqueue_substep(World& w, Scene* ds, const RefOut& ro, bool t
             w.launches++;
         }
         if (v.ntiles > kScanTiles) {
-            k_tiles_list<<<cdiv(v.ntiles, 1024), 1024, 0, st>>>(v);
-            w.launches++;
+            const uint32_t groups = cdiv(v.ntiles, 1024);
+            k_tiles_sum<<<groups, 1024, 0, st>>>(v);
+            k_tiles_list<<<groups, 1024, 0, st>>>(v);
+            w.launches += 2;
         }
         k_bin_cells<<<w.bin_blocks, kTileCells, 0, st>>>(v);
         // it takes the positions and the tiles: blocks for whichever are more (with

@@ -86,6 +86,7 @@ struct WorldView {
     uint4* chunk_hdr;          // per chunk of this substep's layout, 2 words: the packed ChunkHdr (written by the binning)
     uint32_t* tile_cnt;        // per tile: particles for the next binning (counted by G2P and imports)
     uint2* tile_base;          // per listed tile: its first position and chunk (worlds of many tiles)
+    uint4* tile_group;         // per 1,024 tiles: their load (two words) and occupied tiles (worlds of many tiles)
     uint32_t* tile_occ_list;
     uint32_t* tile_grid_list;
     Ctrl* ctrl;
@@ -201,6 +202,7 @@ struct World {
     uint32_t* tile_flags = nullptr;
     uint32_t* tile_cnt = nullptr;
     uint2* tile_base = nullptr;
+    uint4* tile_group = nullptr;
     uint4* chunk_hdr = nullptr;
     uint32_t chunk_cap = 0;
     uint32_t chunk = kChunk;   // chunk size of the substep being enqueued
