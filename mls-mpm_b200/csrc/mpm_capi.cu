@@ -200,8 +200,8 @@ static cudaError_t sync_reference_buffers(Scene& s, uint32_t which = kParticleSt
 }
 
 // Turns on the substeps' own writes of pos, vel and density in the reference
-// layout.  Large scenes get k_mirror's table here; without memory for it G2P
-// goes on writing the buffers, as it does in smaller scenes.
+// layout.  Scenes that can grow large enough get k_mirror's table here; without
+// memory for it G2P goes on writing the buffers, as it does in smaller scenes.
 static void start_mirror(Scene& s) {
     s.mirror = true;
     if (s.capacity < kMirrorGather) return;

@@ -79,8 +79,8 @@ struct DiffuseState {
 // substep (MPM_FLAG_PLAIN), which mirrors the reference's dispatch list.
 enum Engine { kEngineBinned = 0, kEnginePlain = 1 };
 
-// Render buffers by k_mirror (mpm_world.cu): scenes of at least this capacity,
-// more than this many substeps after their load.
+// Render buffers by k_mirror (mpm_world.cu): scenes of at least this many active
+// particles, more than this many substeps after their load.
 #ifndef MPM_MIRROR_GATHER
 #define MPM_MIRROR_GATHER 1500000
 #endif

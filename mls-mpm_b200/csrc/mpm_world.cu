@@ -2045,8 +2045,8 @@ __global__ void __launch_bounds__(kChunkThreads, MPM_G2P_MINB) k_g2p_chunks(Worl
 // stays in L2.  G2P with the buffers kept by its own writes / by this pass, us,
 // 5, 60 and 300 substeps after the load: 1M 65 78 67 / 77 87 73, 1.7M 99 120 135 /
 // 115 132 120, 2.5M 137 180 219 / 162 177 167, 8.4M 432 609 870 / 499 545 570.  So
-// it runs in scenes of kMirrorGather particles from kMirrorMixed substeps after
-// their load on.
+// it runs in scenes of kMirrorGather active particles or more (whatever their
+// capacity), from kMirrorMixed substeps after their load on.
 __global__ void __launch_bounds__(256) k_mirror(RefOut ro, uint32_t n) {
     constexpr uint32_t kPer = 4;   // records in flight a thread
     const uint32_t i0 = blockIdx.x * (256u * kPer) + threadIdx.x;
@@ -2641,7 +2641,8 @@ cudaError_t world_substep(World& w, Scene* ds, bool use_graph) {
         ro.dens = ds->dens;
         // the records go where the old rows were: P2G_MOM has read them, and the
         // next substep's G2P writes that buffer anew
-        if (ds->mirror_where && ds->substeps_done - ds->loaded_at > kMirrorMixed) {
+        if (ds->mirror_where && w.scenes[ds->world_slot].n >= kMirrorGather &&
+            ds->substeps_done - ds->loaded_at > kMirrorMixed) {
             ro.record = w.rows[w.cur];
             ro.where = ds->mirror_where;
         }
