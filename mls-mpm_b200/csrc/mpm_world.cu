@@ -2547,9 +2547,12 @@ static cudaError_t enqueue_substep(World& w, Scene* ds, const RefOut& ro, bool t
         w.launches++;
     }
     // A launch less is worth more than decoding every staged halo until blocks
-    // take a second chunk: frame of 8k particles 13.6 -> 12.7 us, 64k 20.2 -> 19.0
-    // (three scenes in turn), but 230k 56.9 -> 58.8.
-    const bool raw_mass = w.chunk == kChunkSmall && w.n_total <= w.item_blocks * kChunkSmall;
+    // take a second chunk, of the four blocks an SM of the default shape: frame of
+    // 8k particles 13.6 -> 12.7 us, 64k 20.2 -> 19.0 (three scenes in turn), but
+    // 230k 56.9 -> 58.8.  More blocks (batches whose shape was tuned) don't move
+    // the line: 30 scenes of 8,000 particles, tuned, 89.0 us, and 90.3 with a line
+    // that followed the shape.
+    const bool raw_mass = w.chunk == kChunkSmall && w.n_total <= std::min(w.item_blocks, w.sms * 4) * kChunkSmall;
     if (!raw_mass) {
         Phase ph(prof, MPM_PHASE_DECODE_MASS);
         k_decode_tiles<<<w.grid_blocks, 256, 0, st>>>(v, cm, w.cmf);
