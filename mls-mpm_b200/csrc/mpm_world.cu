@@ -402,9 +402,8 @@ struct ChunkHdr {
     int32_t hx, hy, hz;      // halo dims
 };
 
-// The box of the local cells [lo, hi] (x fastest, then y, then z) plus one
-// cell on every side.
-// The box of a chunk of tile (tx, ty, tz) of `scene` whose cells go from lo to hi.
+// The box of a chunk of tile (tx, ty, tz) of `scene` whose local cells (x fastest,
+// then y, then z) go from lo to hi: a box that holds them, plus one cell on every side.
 __device__ __forceinline__ void chunk_header_from(uint32_t scene, uint32_t tx, uint32_t ty, uint32_t tz, uint32_t lo,
                                                   uint32_t hi, ChunkHdr& h) {
     constexpr uint32_t kRow = kTileX, kSlab = kTileX * kTileY;
@@ -598,7 +597,7 @@ __device__ __forceinline__ void tile_grid_entry(const WorldView& v, uint32_t t) 
 // perm[new position] = previous position for every particle, and the
 // grid-tile list.  Also advances the diffuse seed (diffuse-gpu.js:149).
 __global__ void k_scatter(WorldView v, mpm_gen_params* gen) {
-    const uint32_t total = v.ctrl->total_pos;   // (of the previous layout: DECODE_MASS sets this one's)
+    const uint32_t total = v.ctrl->total_pos;   // (of the previous layout: P2G_MASS sets this one's)
     const uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
     if (i0 == 0 && gen) gen->seed = gen->seed + 1u;
     for (uint32_t t = i0; t < v.ntiles; t += stride) tile_grid_entry(v, t);
@@ -687,7 +686,7 @@ __device__ __forceinline__ float2 sadd(float2 a, float2 b) { return make_float2(
 // ---------------------------------------------------------------------------
 // Chunks in shared memory
 // ---------------------------------------------------------------------------
-// Chunks of the layout of parity p.
+// Chunks of this substep's layout.
 __device__ __forceinline__ uint32_t chunk_count(const WorldView& v) {
     return min(v.ctrl->n_chunks, v.chunk_cap);
 }
@@ -2519,7 +2518,7 @@ static cudaError_t enqueue_substep(World& w, Scene* ds, const RefOut& ro, bool t
     {
         Phase ph(prof, MPM_PHASE_SORT);
         if (!w.counted) {
-            // nothing counted yet (a new world, or positions edited in place): count all
+            // nothing counted yet (a new world): count all
             e = cudaMemsetAsync(w.cell_count, 0, ((size_t)w.cell_cap + 1) * 4, st);
             if (e != cudaSuccess) return e;
             k_count<<<nposb, 256, 0, st>>>(v);
@@ -2669,11 +2668,15 @@ cudaError_t world_substep(World& w, Scene* ds, bool use_graph) {
     }
     const bool tail_in = diffuse && ds->diffuse.tail_pending;
     const bool defer = diffuse && !profiling;
-    // Capturing and instantiating a substep costs the host about 0.2 ms a graph
-    // (two parities), launching its kernels one by one about 20 us more than
-    // replaying: a graph pays off once its launch arguments last some
-    // kCaptureAfter substeps.  Worlds whose scenes change every few substeps
-    // (an editing user, a serving loop) are never captured.
+    // Capturing and instantiating a substep costs the host 0.13 to 0.17 ms a graph
+    // (two parities); its kernels launched one by one take 40 us a substep at 8k
+    // particles, where a replay takes 30, and as long as a replay from 300k on.  So a
+    // graph pays off once its launch arguments last some kCaptureAfter substeps.  The
+    // first 1, 16 and 80 substeps after a load, ms: 8k 0.06 0.64 2.56 (captured at once
+    // 0.20 0.73 2.64, after 40 substeps 0.06 0.64 2.80), 300k 0.11 1.34 6.38 (0.28 1.39
+    // 6.43; 0.11 1.34 6.64), 1M 0.24 3.06 15.6 (0.44 3.04 15.6; 0.24 3.05 15.9).
+    // Worlds whose scenes change every few substeps (an editing user) are never
+    // captured.
     constexpr uint32_t kCaptureAfter = 16;
     if (w.generation_seen != w.generation) {
         w.generation_seen = w.generation;

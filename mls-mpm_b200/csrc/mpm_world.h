@@ -159,9 +159,11 @@ struct World {
     int gbuf = 0;                           // i32 grid buffer the next substep accumulates into
     bool dens_valid = false;
     bool table_dirty = true;
-    // true when the last substep's G2P left every position's rank within its
-    // binning cell in rank/cell_count; adding or removing a scene clears it
-    // and the next substep recounts (k_count)
+    // false only before the first substep, which counts every position's cell
+    // (k_count); afterwards G2P leaves every rank within its cell in rank /
+    // cell_count, and adding or removing a scene counts that scene alone.  The
+    // tiles' counts (tile_cnt) are kept by imports, removals and G2P throughout:
+    // whoever clears this flag has to recount them too.
     bool counted = false;
     bool dense = false;   // the layout is the last substep's: no holes, scenes in the order of their tiles
     uint64_t launches = 0;
@@ -260,7 +262,7 @@ struct Scene;
 // One substep of every scene.  owner: the single-scene wrapper of a world of
 // one scene (its diffuse pool and reference-layout mirrors follow that scene;
 // null for batches).  use_graph: replay a captured CUDA graph of the substep
-// (captured on first use and whenever the scene set changes).
+// (captured once its launch arguments have lasted some substeps).
 cudaError_t world_substep(World& w, Scene* owner, bool use_graph);
 // Runs the owner's deferred diffuse tail now, in stream order (no-op when
 // none is pending).
